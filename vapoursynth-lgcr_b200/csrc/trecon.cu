@@ -9,6 +9,7 @@
 // confidence by its chroma consistency. Workspaces for those stages are
 // pooled per filter.
 #include "impl.h"
+#include "temporal.cuh"
 #include "trecon.h"
 
 #include <algorithm>
@@ -49,7 +50,14 @@ struct lgcr_trecon {
     int trad = 1, tsearch = 6, numFrames = 0;
     double tsad = 0.02;
     float nw[2][129] = {};              // phase-novelty factors per axis, mv + 64
-    float *dNw = nullptr;               // their device copy (first frame call)
+    // device tables (first frame call): the novelty factors, then the lanczos
+    // factors of both axes as doubles
+    float *dNw = nullptr;
+    static constexpr size_t kLanOffset = (sizeof(float) * 2 * 129 + 255) & ~size_t(255);
+    const double *deviceLan(int axis) const {
+        return reinterpret_cast<const double *>(reinterpret_cast<const char *>(dNw) + kLanOffset) +
+               axis * kTLanEntries;
+    }
     std::mutex mu;
     std::vector<std::unique_ptr<TReconWorkspace>> idle;
     ~lgcr_trecon() {
@@ -60,14 +68,22 @@ struct lgcr_trecon {
     const float *deviceNw() {
         std::lock_guard<std::mutex> lock(mu);
         if (!dNw) {
-            float *p = nullptr;
-            if (cudaMalloc(&p, sizeof(nw)) != cudaSuccess)
+            char *p = nullptr;
+            if (cudaMalloc(&p, kLanOffset + 2 * kTLanEntries * sizeof(double)) != cudaSuccess)
                 return nullptr;
-            if (cudaMemcpy(p, nw, sizeof(nw), cudaMemcpyHostToDevice) != cudaSuccess) {
+            const Filter &F = *filter;
+            double *lan = reinterpret_cast<double *>(p + kLanOffset);
+            const double rw = double(F.sw) / F.cw, rh = double(F.sh) / F.ch;
+            const cudaStream_t s = callingThreadStream();
+            // the scale factors buildJob gives the frame (same-size output)
+            launchTReconLanczos(lan, lan + kTLanEntries, rw, rh, float(std::min(1.0, double(F.sw) / F.cw)),
+                                float(std::min(1.0, double(F.sh) / F.ch)), F.p.k.support, s);
+            if (cudaMemcpy(p, nw, sizeof(nw), cudaMemcpyHostToDevice) != cudaSuccess ||
+                cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
                 cudaFree(p);
                 return nullptr;
             }
-            dNw = p;
+            dNw = reinterpret_cast<float *>(p);
         }
         return dNw;
     }
@@ -382,6 +398,8 @@ int lgcr_trecon_frame(lgcr_trecon *t, const lgcr_plane cur[3], const lgcr_plane 
         J.tnbCount = count;
         J.tnwX = dNw;
         J.tnwY = dNw + 129;
+        J.tlanX = t->deviceLan(0);
+        J.tlanY = t->deviceLan(1);
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(ws->dJob, ws->hJob, sizeof(FrameJob), cudaMemcpyHostToDevice, s);

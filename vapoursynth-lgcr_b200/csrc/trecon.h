@@ -33,6 +33,11 @@ struct TReconPrep {
     const int *lcXb, *lcXe, *lcYb, *lcYe;   // footprint extents at the frame's siting
 };
 
+// Fills the lanczos factor tables of the temporal taps (kTLanEntries per
+// axis, temporal.cuh) on `s`.
+void launchTReconLanczos(double *tabX, double *tabY, double rw, double rh, float invWx, float invWy,
+                         double support, cudaStream_t s);
+
 // Enqueues conversion, footprint maps, block matching and the consistency
 // check for neighbours 1 .. frames - 1. Returns the number of launches, or
 // -1 when a launch failed.
