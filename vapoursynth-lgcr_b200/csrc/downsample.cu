@@ -55,6 +55,43 @@ WeightTable downsampleWeights(int srcN, int kernel, float shift) {
     return buildWeights(srcN, srcN / 2, k, shift);
 }
 
+// Spatial weights of every window tap and envelope (kDsSlots) and the window's
+// place; the float expressions and their order are spatialWeight's.
+struct SpatialTable {
+    std::vector<float> w;
+    int x0 = 0, y0 = 0, width = 0, height = 0;
+};
+
+SpatialTable spatialTable(int quality, float shiftX, float shiftY) {
+    static const float dir[8][2] = {{1.0f, 0.0f}, {0.9238795f, 0.3826834f}, {0.7071068f, 0.7071068f},
+                                    {0.3826834f, 0.9238795f}, {0.0f, 1.0f}, {-0.3826834f, 0.9238795f},
+                                    {-0.7071068f, 0.7071068f}, {-0.9238795f, 0.3826834f}};
+    const int radius = quality == 0 ? 2 : quality == 1 ? 3 : 4;
+    const float fx = 0.5f + shiftX, fy = 0.5f + shiftY;
+    SpatialTable t;
+    t.x0 = int(std::ceil(fx - radius));
+    t.y0 = int(std::ceil(fy - radius));
+    t.width = int(std::floor(fx + radius)) - t.x0 + 1;
+    t.height = int(std::floor(fy + radius)) - t.y0 + 1;
+    t.w.assign(size_t(t.width) * t.height * kDsSlots, 0.0f);
+    for (int j = 0; j < t.height; ++j)
+        for (int i = 0; i < t.width; ++i) {
+            const float dx = float(t.x0 + i) - fx, dy = float(t.y0 + j) - fy;
+            const float radius2 = dx * dx + dy * dy;
+            float *w = &t.w[size_t(j * t.width + i) * kDsSlots];
+            for (int set = 0; set < 2; ++set) {
+                const float anisotropy = set ? 2.7f : quality == 0 ? 1.8f : 2.2f;
+                for (int d = 0; d < 8; ++d) {
+                    const float nd = dx * dir[d][0] + dy * dir[d][1];
+                    const float td = -dx * dir[d][1] + dy * dir[d][0];
+                    w[set * 9 + d] = 1.0f / (1.0f + (0.9f + anisotropy) * nd * nd + 0.16f * td * td);
+                }
+                w[set * 9 + 8] = 1.0f / (1.0f + 0.42f * radius2);
+            }
+        }
+    return t;
+}
+
 struct DsWorkspace {
     DeviceArena arena;
     float2 *rows = nullptr;
@@ -78,7 +115,8 @@ struct lgcr_downsample {
     DeviceArena tables;
     int hSup = 0, vSup = 0;
     const int *hStart = nullptr, *vStart = nullptr;
-    const float *hW = nullptr, *vW = nullptr;
+    const float *hW = nullptr, *vW = nullptr, *spatial = nullptr;
+    SpatialTable window;
     std::mutex mu;
     std::vector<std::unique_ptr<DsWorkspace>> idle;
 
@@ -200,11 +238,14 @@ int lgcr_downsample_create(const lgcr_downsample_params *params, const lgcr_form
     const WeightTable ty = downsampleWeights(fmt->height, d->kernel, d->shiftY);
     const size_t oHs = d->tables.reserve(tx.start.size() * 4), oHw = d->tables.reserve(tx.w.size() * 4);
     const size_t oVs = d->tables.reserve(ty.start.size() * 4), oVw = d->tables.reserve(ty.w.size() * 4);
+    d->window = spatialTable(d->quality, d->shiftX, d->shiftY);
+    const size_t oSp = d->tables.reserve(d->window.w.size() * 4);
     if (!d->tables.commit())
         return fail("Downsample: device table allocation failed", LGCR_E_NOMEM);
-    const struct { size_t off; const void *src; size_t bytes; } up[4] = {
+    const struct { size_t off; const void *src; size_t bytes; } up[5] = {
         {oHs, tx.start.data(), tx.start.size() * 4}, {oHw, tx.w.data(), tx.w.size() * 4},
-        {oVs, ty.start.data(), ty.start.size() * 4}, {oVw, ty.w.data(), ty.w.size() * 4}};
+        {oVs, ty.start.data(), ty.start.size() * 4}, {oVw, ty.w.data(), ty.w.size() * 4},
+        {oSp, d->window.w.data(), d->window.w.size() * 4}};
     for (const auto &u : up)
         if (cudaMemcpy(d->tables.at(u.off), u.src, u.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
             return fail("Downsample: table upload failed", LGCR_E_CUDA);
@@ -214,6 +255,7 @@ int lgcr_downsample_create(const lgcr_downsample_params *params, const lgcr_form
     d->hW = (const float *)d->tables.at(oHw);
     d->vStart = (const int *)d->tables.at(oVs);
     d->vW = (const float *)d->tables.at(oVw);
+    d->spatial = (const float *)d->tables.at(oSp);
     *out = d.release();
     return LGCR_OK;
 }
@@ -298,6 +340,9 @@ int lgcr_downsample_frame(lgcr_downsample *d, const lgcr_plane in[3], const lgcr
     J.strength = d->strength;
     J.shiftX = d->shiftX;
     J.shiftY = d->shiftY;
+    J.spatial = d->spatial;
+    J.winX0 = d->window.x0; J.winY0 = d->window.y0;
+    J.winW = d->window.width; J.winH = d->window.height;
     if (e == cudaSuccess)
         e = launchDownsample(J, st);
     // luma: the reference shares the source's Y plane with its output frame

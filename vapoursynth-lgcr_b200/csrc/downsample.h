@@ -14,6 +14,16 @@ enum DsCandidatePlane : int {
     kDsBaseU = 0, kDsBaseV = 1, kDsGate = 2, kDsCandU = 3, kDsCandV = 7, kDsPlanes = 11
 };
 
+// Spatial weights of the guided windows (spatialWeight,
+// src/downsample.cpp:393-402). The window of an output sample lies at the
+// same offsets from its centre everywhere (centre 2x + 0.5 + shift, exact in
+// float), so a weight depends on the tap and on the envelope's direction
+// only: [tap of the window, rows then columns][kDsSlots], slots 0-7 the
+// directions and 8 the isotropic envelope of the smaller radius, 9-16 and 17
+// those of quality 2's larger one.
+constexpr int kDsSlots = 18;
+constexpr int kDsMaxTaps = 81;
+
 struct DownsampleJob {
     int W, H;                           // source (4:4:4) size, both even
     int cw, ch;                         // output chroma size W / 2, H / 2
@@ -32,6 +42,8 @@ struct DownsampleJob {
     float *cand;                        // kDsPlanes x cw x ch (quality 2)
     int quality;
     float strength, shiftX, shiftY;
+    const float *spatial;               // winW * winH * kDsSlots
+    int winX0, winY0, winW, winH;       // window of output (x, y): first sample 2x + winX0, 2y + winY0
 };
 
 cudaError_t launchDownsample(const DownsampleJob &J, cudaStream_t s);

@@ -17,8 +17,7 @@
 //               keeps the best (scoreCandidateRow, 577-651).
 // All arithmetic is FP32 in the reference's order (the library is compiled
 // without FMA contraction), with its clamped sample reads; quotients are
-// IEEE divisions, or the reciprocal refinement equal to them on [1, 2^64)
-// where the denominator is 1 plus a non-negative term.
+// IEEE divisions or refinements equal to them.
 #include "downsample.h"
 
 namespace lgcr_b200 {
@@ -190,58 +189,61 @@ __device__ DsStats dsClassify(const DsTile &T, float centerX, float centerY, int
     return st;
 }
 
-struct DsEnvelope {
-    DsDirection normal;
-    int radius;
-    float anisotropy;
-    bool isotropic;
-};
-
-// spatialWeight (downsample.cpp:393-402); denominators are 1 plus
-// non-negative terms of offsets within 4 samples
-__device__ __forceinline__ float dsSpatial(const DsEnvelope &e, float dx, float dy) {
-    const float radius2 = dx * dx + dy * dy;
-    if (e.isotropic)
-        return rcpInRange(1.0f + 0.42f * radius2);
-    const float nd = dx * e.normal.x + dy * e.normal.y;
-    const float td = -dx * e.normal.y + dy * e.normal.x;
-    return rcpInRange(1.0f + (0.9f + e.anisotropy) * nd * nd + 0.16f * td * td);
+// kDsRangeScale2 / d for kDsRangeScale2 <= d: a refined reciprocal and
+// Markstein's remainder step (IBM J. Res. Dev. 34(1), 1990), the IEEE
+// quotient for finite d; float formats, whose d may overflow, divide.
+template <int KIND>
+__device__ __forceinline__ float dsRange(float d) {
+    if (KIND == kF32)
+        return kDsRangeScale2 / d;
+    const float r = rcpInRange(d);
+    const float q = kDsRangeScale2 * r;
+    return __fmaf_rn(__fmaf_rn(-q, d, kDsRangeScale2), r, q);
 }
 
 // accumulateGuided (downsample.cpp:404-451): range- and spatially-weighted
-// sums of U and V over the envelopes' common window, per envelope
-template <int N>
-__device__ __forceinline__ void dsAccumulate(const DsTile &T, float centerX, float centerY,
-                                             const DsEnvelope (&env)[N], float (&aw)[N],
-                                             float (&au)[N], float (&av)[N]) {
-    int maxRadius = 0;
+// sums of U and V over the envelopes' common window, per envelope. sW: the
+// block's copy of the spatial table; slot[i]: envelope i's column of it. The
+// first SMALL envelopes end at radius 3 of quality 2's window of radius 4 (a
+// test of the tap, the same for the whole block).
+//
+// Bound by issue: with the spatial weights evaluated per tap and envelope
+// (about 14 instructions each) this loop was three quarters of the kernel;
+// read from the table it is one shared load. 1080p 10-bit quality 2:
+// k_ds_pixel 223 -> 104 us.
+template <int KIND, int N, int SMALL>
+__device__ __forceinline__ void dsAccumulate(const DownsampleJob &J, const DsTile &T, const float *sW, int x,
+                                             int y, float centerX, float centerY, const int (&slot)[N],
+                                             float (&aw)[N], float (&au)[N], float (&av)[N]) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        maxRadius = max(maxRadius, env[i].radius);
+    for (int i = 0; i < N; ++i)
         aw[i] = au[i] = av[i] = 0.0f;
-    }
-    const int x0 = (int)ceilf(centerX - maxRadius), x1 = (int)floorf(centerX + maxRadius);
-    const int y0 = (int)ceilf(centerY - maxRadius), y1 = (int)floorf(centerY + maxRadius);
     const int cx0 = (int)floorf(centerX), cy0 = (int)floorf(centerY);
     const float fx = centerX - cx0, fy = centerY - cy0;
     const float ya = T.Y(cx0, cy0), yb = T.Y(cx0 + 1, cy0);
     const float yc = T.Y(cx0, cy0 + 1), yd = T.Y(cx0 + 1, cy0 + 1);
     const float centerLuma = ya + (yb - ya) * fx + (yc - ya) * fy + (ya - yb - yc + yd) * fx * fy;
-    for (int sy = y0; sy <= y1; ++sy) {
-        for (int sx = x0; sx <= x1; ++sx) {
-            const float dx = sx - centerX, dy = sy - centerY;
-            const int o = T.idx(sx, sy);
+    const int x0 = 2 * x + J.winX0, y0 = 2 * y + J.winY0;
+    const float *w = sW;
+    for (int j = 0; j < J.winH; ++j) {
+        // |dy| <= 3 (dy = winY0 + j - fraction of the centre)
+        const bool rowIn = SMALL == 0 || fabsf((float)(J.winY0 + j) - (0.5f + J.shiftY)) <= 3.0f;
+        const int row = T.idx(x0, y0 + j);
+        for (int i = 0; i < J.winW; ++i, w += kDsSlots) {
+            const int o = row + i;
             const float delta = T.y[o] - centerLuma;
-            const float rangeWeight = kDsRangeScale2 / (kDsRangeScale2 + delta * delta);
+            const float rangeWeight = dsRange<KIND>(kDsRangeScale2 + delta * delta);
             const float su = T.u[o], sv = T.v[o];
+            const bool in = SMALL == 0 ||
+                (rowIn && fabsf((float)(J.winX0 + i) - (0.5f + J.shiftX)) <= 3.0f);
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-                if (fabsf(dx) > env[i].radius || fabsf(dy) > env[i].radius)
+            for (int e = 0; e < N; ++e) {
+                if (e < SMALL && !in)
                     continue;
-                const float weight = rangeWeight * dsSpatial(env[i], dx, dy);
-                aw[i] += weight;
-                au[i] += weight * su;
-                av[i] += weight * sv;
+                const float weight = rangeWeight * w[slot[e]];
+                aw[e] += weight;
+                au[e] += weight * su;
+                av[e] += weight * sv;
             }
         }
     }
@@ -274,6 +276,7 @@ template <int KIND, bool GUIDED>
 __global__ void __launch_bounds__(256) k_ds_pixel(DownsampleJob J) {
     __shared__ float sY[GUIDED ? kDsTw * kDsTh : 1], sU[GUIDED ? kDsTw * kDsTh : 1],
         sV[GUIDED ? kDsTw * kDsTh : 1];
+    __shared__ float sW[GUIDED ? kDsMaxTaps * kDsSlots : 1];
     const int bx0 = blockIdx.x * kDsBx, by0 = blockIdx.y * kDsBy;
     const int x = bx0 + threadIdx.x, y = by0 + threadIdx.y;
     const bool inside = x < J.cw && y < J.ch;
@@ -303,6 +306,8 @@ __global__ void __launch_bounds__(256) k_ds_pixel(DownsampleJob J) {
         sU[k] = dsLoad<KIND>(J, 1, sx, sy);
         sV[k] = dsLoad<KIND>(J, 2, sx, sy);
     }
+    for (int k = threadIdx.y * kDsBx + threadIdx.x; k < J.winW * J.winH * kDsSlots; k += kDsBx * kDsBy)
+        sW[k] = __ldg(J.spatial + k);
     __syncthreads();
     if (!inside)
         return;
@@ -316,16 +321,15 @@ __global__ void __launch_bounds__(256) k_ds_pixel(DownsampleJob J) {
         if (st.gate <= kDsActivation) {
             gate = 0.0f;
         } else if (J.quality == 0) {
-            const DsEnvelope env[1] = {{kDsDirections[st.primary], 2, 1.8f, st.isotropic}};
+            const int slot[1] = {st.isotropic ? 8 : st.primary};
             float aw[1], au[1], av[1];
-            dsAccumulate<1>(T, centerX, centerY, env, aw, au, av);
+            dsAccumulate<KIND, 1, 0>(J, T, sW, x, y, centerX, centerY, slot, aw, au, av);
             gu = dsNorm(au[0], aw[0], bu);
             gv = dsNorm(av[0], aw[0], bv);
         } else {
-            const DsEnvelope env[2] = {{kDsDirections[st.primary], 3, 2.2f, st.isotropic},
-                                       {kDsDirections[st.secondary], 3, 2.2f, st.isotropic}};
+            const int slot[2] = {st.isotropic ? 8 : st.primary, st.isotropic ? 8 : st.secondary};
             float aw[2], au[2], av[2];
-            dsAccumulate<2>(T, centerX, centerY, env, aw, au, av);
+            dsAccumulate<KIND, 2, 0>(J, T, sW, x, y, centerX, centerY, slot, aw, au, av);
             const float u0 = dsNorm(au[0], aw[0], bu), v0 = dsNorm(av[0], aw[0], bv);
             const float u1 = dsNorm(au[1], aw[1], bu), v1 = dsNorm(av[1], aw[1], bv);
             gu = u0 + st.secondaryMix * (u1 - u0);
@@ -351,15 +355,10 @@ __global__ void __launch_bounds__(256) k_ds_pixel(DownsampleJob J) {
         }
         return;
     }
-    const DsEnvelope env[5] = {
-        {kDsDirections[st.primary], 3, 2.2f, st.isotropic},
-        {kDsDirections[st.secondary], 3, 2.2f, st.isotropic},
-        {kDsDirections[st.primary], 4, 2.7f, st.isotropic},
-        {kDsDirections[st.secondary], 4, 2.7f, st.isotropic},
-        {kDsDirections[st.primary], 4, 0.0f, true},
-    };
+    const int first = st.isotropic ? 8 : st.primary, second = st.isotropic ? 8 : st.secondary;
+    const int slot[5] = {first, second, 9 + first, 9 + second, 17};
     float aw[5], au[5], av[5];
-    dsAccumulate<5>(T, centerX, centerY, env, aw, au, av);
+    dsAccumulate<KIND, 5, 2>(J, T, sW, x, y, centerX, centerY, slot, aw, au, av);
     const float u0 = dsNorm(au[0], aw[0], bu), v0 = dsNorm(av[0], aw[0], bv);
     const float u1 = dsNorm(au[1], aw[1], bu), v1 = dsNorm(av[1], aw[1], bv);
     C[kDsCandU * plane] = u0 + st.secondaryMix * (u1 - u0);
@@ -373,17 +372,41 @@ __global__ void __launch_bounds__(256) k_ds_pixel(DownsampleJob J) {
 
 // scoreCandidateRow (downsample.cpp:571-651): re-upsample each candidate
 // bilinearly to the sample's four source positions, keep the lowest
-// edge-weighted squared error
+// edge-weighted squared error. The block blends the candidates of its tile and
+// one sample around it once into shared memory (the four positions read each
+// neighbour up to four times, and its gate, base and candidates from eleven
+// planes): 1080p 52 -> 32 us.
+constexpr int kDsSw = kDsBx + 2, kDsSh = kDsBy + 2;
+
 template <int KIND>
 __global__ void __launch_bounds__(256) k_ds_score(DownsampleJob J) {
-    const int x = blockIdx.x * kDsBx + threadIdx.x, y = blockIdx.y * kDsBy + threadIdx.y;
-    if (x >= J.cw || y >= J.ch)
-        return;
+    __shared__ float2 sC[4][kDsSh][kDsSw];             // blended (U, V) of each candidate
+    const int bx0 = blockIdx.x * kDsBx, by0 = blockIdx.y * kDsBy;
+    const int x = bx0 + threadIdx.x, y = by0 + threadIdx.y;
+    const bool inside = x < J.cw && y < J.ch;
     const size_t plane = (size_t)J.cw * J.ch;
     const float *C = J.cand;
     const size_t o = (size_t)y * J.cw + x;
+    float gate = 0.0f;
+    if (inside)
+        gate = C[kDsGate * plane + o];
+    if (__syncthreads_or(gate != 0.0f)) {
+        for (int k = threadIdx.y * kDsBx + threadIdx.x; k < kDsSw * kDsSh; k += kDsBx * kDsBy) {
+            const int r = k / kDsSw, c = k - r * kDsSw;
+            // samples beyond the plane's edge stand for the clamped ones
+            const size_t at = (size_t)iclamp(by0 - 1 + r, 0, J.ch - 1) * J.cw + iclamp(bx0 - 1 + c, 0, J.cw - 1);
+            const float g = C[kDsGate * plane + at];
+            const float vu = C[kDsBaseU * plane + at], vv = C[kDsBaseV * plane + at];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                sC[q][r][c] = make_float2(vu + g * (C[(kDsCandU + q) * plane + at] - vu),
+                                          vv + g * (C[(kDsCandV + q) * plane + at] - vv));
+        }
+        __syncthreads();
+    }
+    if (!inside)
+        return;
     const float bu = C[kDsBaseU * plane + o], bv = C[kDsBaseV * plane + o];
-    const float gate = C[kDsGate * plane + o];
     if (gate == 0.0f) {
         dsStore(J, 0, x, y, bu);
         dsStore(J, 1, x, y, bv);
@@ -400,24 +423,18 @@ __global__ void __launch_bounds__(256) k_ds_score(DownsampleJob J) {
             const float lowY = (hy - 0.5f - J.shiftY) * 0.5f;
             const float sourceU = dsLoad<KIND>(J, 1, hx, hy), sourceV = dsLoad<KIND>(J, 2, hx, hy);
             const int rawX0 = (int)floorf(lowX), rawY0 = (int)floorf(lowY);
-            const int xa = iclamp(rawX0, 0, J.cw - 1), xb = iclamp(rawX0 + 1, 0, J.cw - 1);
-            const int ra = iclamp(rawY0, 0, J.ch - 1), rb = iclamp(rawY0 + 1, 0, J.ch - 1);
             const float fx = lowX - rawX0, fy = lowY - rawY0;
             const float wts[4] = {(1.0f - fx) * (1.0f - fy), fx * (1.0f - fy), (1.0f - fx) * fy, fx * fy};
-            const size_t at[4] = {(size_t)ra * J.cw + xa, (size_t)ra * J.cw + xb,
-                                  (size_t)rb * J.cw + xa, (size_t)rb * J.cw + xb};
+            const int cx = rawX0 - bx0 + 1, cy = rawY0 - by0 + 1;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
+                const float2 a = sC[c][cy][cx], b = sC[c][cy][cx + 1];
+                const float2 d = sC[c][cy + 1][cx], e = sC[c][cy + 1][cx + 1];
                 float ru = 0.0f, rv = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float g = C[kDsGate * plane + at[k]];
-                    float vu = C[kDsBaseU * plane + at[k]], vv = C[kDsBaseV * plane + at[k]];
-                    vu += g * (C[(kDsCandU + c) * plane + at[k]] - vu);
-                    vv += g * (C[(kDsCandV + c) * plane + at[k]] - vv);
-                    ru += wts[k] * vu;
-                    rv += wts[k] * vv;
-                }
+                ru += wts[0] * a.x; rv += wts[0] * a.y;
+                ru += wts[1] * b.x; rv += wts[1] * b.y;
+                ru += wts[2] * d.x; rv += wts[2] * d.y;
+                ru += wts[3] * e.x; rv += wts[3] * e.y;
                 const float du = ru - sourceU, dv = rv - sourceV;
                 scores[c] += edgeWeight * (du * du + dv * dv);
             }
