@@ -233,7 +233,7 @@ __device__ __forceinline__ void convertChroma(const FrameJob &J, int cy, int xb,
                         for (int i = xb0; i < xe0; ++i)
                             sum += (double)rawToFloat<KIND>(rawLoad<KIND>(lrow, i), scale, 0.0);
                 }
-                lc[o] = (float)(sum / ((double)(xe0 - xb0) * (double)(ye - yb)));
+                lc[o] = footprintMean(sum, xe0 - xb0, ye - yb);
             }
         }
     }

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) k_trecon_lc(const TReconPrep P) {
         for (int j = yb; j < ye; ++j)
             for (int x = xb; x < xe; ++x)
                 sum += (double)ldf(Y + (size_t)j * P.sw + x);
-        lc[(size_t)cy * P.cw + cx] = (float)(sum / ((double)(xe - xb) * (double)(ye - yb)));
+        lc[(size_t)cy * P.cw + cx] = footprintMean(sum, xe - xb, ye - yb);
     }
 }
 

@@ -358,6 +358,20 @@ __device__ __forceinline__ float4 bilinearFast4(const float4 *p, int w, int h, i
     return bl4(__ldg(r0), __ldg(r0 + 1), __ldg(r1), __ldg(r1 + 1), fx, fy);
 }
 
+// Mean of a footprint sum (buildLcMap): the usual counts of one, two and four
+// samples are powers of two, whose quotient is an exact product; the FP64
+// division is some forty instructions.
+__device__ __forceinline__ float footprintMean(double sum, int nx, int ny) {
+    const int n = nx * ny;
+    if (n == 4)
+        return (float)(sum * 0.25);
+    if (n == 2)
+        return (float)(sum * 0.5);
+    if (n == 1)
+        return (float)sum;
+    return (float)(sum / ((double)nx * (double)ny));
+}
+
 struct TensorDir { float coherence, nx, ny; };
 
 // lgcr.h:516-538

@@ -239,7 +239,9 @@ int lgcr_sharpen_frame(lgcr_sharpen *s, const lgcr_plane in[3], const lgcr_plane
     J.alpha = float(s->alpha);
     J.sigma = float(s->sigma);
     J.sratio = float(s->sratio);
-    J.invG2 = 1.0f / float(s->gspatial * s->gspatial);
+    const float invG2 = 1.0f / float(s->gspatial * s->gspatial);
+    for (int r2 = 0; r2 < 9; ++r2)
+        J.spatial[r2] = 1.0f / (1.0f + float(r2) * invG2);
     J.margin = float(s->ar);
     J.clampHull = s->ar >= 0.0;
     J.guided = guided;

@@ -19,7 +19,8 @@ struct SharpenJob {
     void *out[3];
     long long outPitch[3];
     float *Ys;                          // sw x sh sharpened luma (chroma guide)
-    float alpha, sigma, sratio, invG2, margin;
+    float alpha, sigma, sratio, margin;
+    float spatial[9];                   // 1 / (1 + r^2 / gspatial^2) by r^2 (1, 2, 4, 5, 8 used)
     int clampHull;                      // ar >= 0
     int guided;                         // chroma subsampled: guided by the luma
     double rw, rh, shiftX, shiftY;      // sw / cw, sh / ch, left siting
