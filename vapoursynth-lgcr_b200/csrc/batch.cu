@@ -143,7 +143,7 @@ struct GroupedPlan {
 };
 
 // groupMode: -1 upscaling frames alone, 0 one group, n >= 1 every n frames
-void planGroups(const std::vector<FrameJob> &jobs, GroupedPlan &gp, int groupMode,
+void planGroups(std::vector<FrameJob> &jobs, GroupedPlan &gp, int groupMode,
                 const LaunchConfig *cfg) {
     const int n = int(jobs.size());
     const int g = groupMode;
@@ -165,6 +165,7 @@ void planGroups(const std::vector<FrameJob> &jobs, GroupedPlan &gp, int groupMod
     const int groups = int(gp.start.size()) - 1;
     gp.plans.resize(groups);
     for (int k = 0; k < groups; ++k) {
+        shapeJobs(jobs.data() + gp.start[k], gp.start[k + 1] - gp.start[k]);
         const std::vector<FrameJob> sub(jobs.begin() + gp.start[k], jobs.begin() + gp.start[k + 1]);
         planStages(sub, gp.plans[k], cfg);
         gp.offset.push_back(gp.offset.back() + gp.plans[k].prefix.size());

@@ -202,6 +202,7 @@ int lgcr_recon_frame(lgcr_recon *h, const lgcr_plane in[3], const lgcr_plane out
     }
     if (e == cudaSuccess) {
         buildJob(t, *ws->hJob);
+        shapeJobs(ws->hJob, 1);
         e = cudaMemcpyAsync(ws->dJob, ws->hJob, sizeof(FrameJob), cudaMemcpyHostToDevice, s);
     }
     if (e == cudaSuccess) {

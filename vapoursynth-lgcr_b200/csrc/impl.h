@@ -165,6 +165,11 @@ void setAxisGeometry(DeviceTables &t, const ChromaAxis &ax, const ChromaAxis &ay
 // Fill the device FrameJob of one task.
 void buildJob(const FrameTask &t, FrameJob &job);
 
+// Work split of the map and plain stages for the frames of one launch (call
+// once for the jobs that are planned and launched together, before they are
+// copied to the device).
+void shapeJobs(FrameJob *jobs, int n);
+
 // Stage scheduler: launches every stage once over all jobs. `dJobs` is the
 // device copy of `jobs`; `dPrefix` receives the stage prefix tables (space
 // for stageCount * (n + 1) ints) and is written from `hPrefix` (pinned,

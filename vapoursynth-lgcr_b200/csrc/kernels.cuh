@@ -37,14 +37,16 @@ __host__ __device__ __forceinline__ int convertLumaBlocks(int sw, int sh) {
 // per strip.
 constexpr int kTensorCols = 28;
 constexpr int kTensorWarps = 8;
-constexpr int kTensorRows = 32;
+constexpr int kTensorRows = 32;        // rows per strip, fewer in small launches (shapeJobs)
 
 // k_dilate_h: widest row in mask words and the zero words on either side
 // (the dilation radius must stay below 32 * kDilPadWords).
 constexpr int kDilMaxWords = 2048;
 constexpr int kDilPadWords = 8;
 
-// k_count: chroma mask bytes per block.
+// k_mark_chroma: list words per warp; k_count: chroma mask bytes per block
+// (256 threads, whole 16-byte vectors). Fewer in small launches (shapeJobs).
+constexpr int kMarkWords = 32;
 constexpr int kCountChunk = 16384;
 
 // k_mark_chroma: output rows per group of an upscaling frame's guided work

@@ -281,7 +281,7 @@ k_convert(LGCR_STAGE_ARGS) {
 // border rule ((2a+b)/9 and (a+2b)/9 at the ends, *(1/9) inside), trust
 // seed jxx + jyy > thr.
 //
-// Each warp walks down a strip of kTensorRows rows over 32 consecutive
+// Each warp walks down a strip of J.tensorRows rows over 32 consecutive
 // columns x0-2 .. x0+29 and emits the 28 middle ones: lane values are luma
 // samples at clamped columns, horizontal neighbours come from shuffles, the
 // three gradient rows and their products roll in registers. The warps of a
@@ -311,8 +311,8 @@ k_tensor(LGCR_STAGE_ARGS) {
     const int x0 = (tile % tilesX) * span + warp * kTensorCols;
     if (x0 >= w)
         return;                                   // whole warp
-    const int y0 = (tile / tilesX) * kTensorRows;
-    const int y1 = min(y0 + kTensorRows, h);
+    const int y0 = (tile / tilesX) * J.tensorRows;
+    const int y1 = min(y0 + J.tensorRows, h);
     const int c = x0 - 2 + lane;
     const bool emitLane = lane >= 2 && lane < 2 + kTensorCols && c < w;
     const float *col = J.Y + iclamp(c, 0, w - 1);
@@ -479,9 +479,9 @@ k_dilate_v(LGCR_STAGE_ARGS) {
 }
 
 // ---------------------------------------------------------------------------
-// Sparse workset: a block covers 256 consecutive 32-pixel words of the
-// output rows in row-group order (markWord); each warp takes 32 of them in
-// turn, one pixel per lane. An output pixel is active when the mask sample
+// Sparse workset: a block covers 8 * J.markWords consecutive 32-pixel words of
+// the output rows in row-group order (markWord); each warp takes J.markWords of
+// them in turn, one pixel per lane. An output pixel is active when the mask sample
 // its position maps to is set (every pixel when the frame is not sparse);
 // active pixels mark the 2x2 chroma bilinear footprint. The block counts its
 // active pixels, takes one range of the frame's guided work list with one
@@ -525,13 +525,14 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
     const int tile = blockIdx.x - tileStart[f];
     const int ow = (J.W + 31) / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wordBase = tile * 256 + warp * 32;          // this warp's 32 words
+    const int per = J.markWords;
+    const int wordBase = (tile * 8 + warp) * per;         // this warp's words
     // pass 1: lane i counts word wordBase + i (and keeps its position for
     // pass 2, where the warp walks the words by shuffles)
     uint32_t myBits = 0;
     int myOy, myKw;
     markWord(wordBase + lane, ow, J.listGroup, myOy, myKw);
-    if (myOy < J.H)
+    if (lane < per && myOy < J.H)
         myBits = activeWord(J, myKw, myOy);
     const unsigned cnt = __popc(myBits);
     unsigned incl = cnt;
@@ -556,7 +557,7 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
     const unsigned excl = incl - cnt;
     const uint32_t below = (1u << lane) - 1u;
     // pass 2: the warp walks its words, one pixel per lane
-    for (int i = 0; i < 32; ++i) {
+    for (int i = 0; i < per; ++i) {
         const uint32_t bits = __shfl_sync(0xffffffffu, myBits, i);
         const unsigned offs = __shfl_sync(0xffffffffu, excl, i);
         if (!bits)
@@ -582,7 +583,7 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
 }
 
 // Active chroma samples: population count of the 0/1 chroma mask bytes, a
-// contiguous 64-byte span per thread, one atomic per block. Frames with a
+// contiguous span of J.countChunk / 256 bytes per thread, one atomic per block. Frames with a
 // chroma work list also get their active samples (y << 16 | x) appended in
 // raster order at the block's range.
 __global__ void __launch_bounds__(256)
@@ -593,12 +594,12 @@ k_count(LGCR_STAGE_ARGS) {
     const FrameJob &J = jobs[f];
     const int tile = blockIdx.x - tileStart[f];
     const size_t nc = (size_t)J.cw * J.ch;
-    const size_t span = (size_t)tile * kCountChunk + (size_t)threadIdx.x * (kCountChunk / 256);
-    const size_t spanEnd = min(nc, span + kCountChunk / 256);
+    const int per = J.countChunk / 256;                    // bytes per thread
+    const size_t span = (size_t)tile * J.countChunk + (size_t)threadIdx.x * per;
+    const size_t spanEnd = min(nc, span + per);
     unsigned c = 0;
-    if (span + kCountChunk / 256 <= nc) {
-#pragma unroll
-        for (int k = 0; k < kCountChunk / 256 / 16; ++k) {
+    if (span + per <= nc) {
+        for (int k = 0; k < per / 16; ++k) {
             const uint4 q = __ldg(reinterpret_cast<const uint4 *>(J.cmask + span) + k);
             c += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
         }

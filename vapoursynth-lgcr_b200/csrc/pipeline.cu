@@ -940,14 +940,14 @@ static int stageTilesShaped(const FrameJob &J, int s) {
     case S_LUMA_RADIAL: return (resize && J.writeLuma && J.radial) ? cdiv(J.W, 32) * cdiv(J.H, 32) : 0;
     case S_LUMA_H: return (resize && J.writeLuma && !J.radial) ? cdiv(J.W, 32) * cdiv(J.sh, 8) : 0;
     case S_LUMA_V: return (resize && J.writeLuma && !J.radial) ? cdiv(J.W, 32) * cdiv(J.H, 8) : 0;
-    case S_TENSOR: return J.guided ? cdiv(J.sw, kTensorCols * kTensorWarps) * cdiv(J.sh, kTensorRows) : 0;
+    case S_TENSOR: return J.guided ? cdiv(J.sw, kTensorCols * kTensorWarps) * cdiv(J.sh, J.tensorRows) : 0;
     case S_DIL_H: return J.sparse ? J.sh : 0;
     case S_DIL_V: return J.sparse ? cdiv(J.maskWords, 32) * cdiv(J.sh, 8) : 0;
     case S_MARK: {
         const int g = std::max(1, J.listGroup);
-        return (J.sparse || J.listed) ? cdiv(cdiv(J.H, g) * g * cdiv(J.W, 32), 256) : 0;
+        return (J.sparse || J.listed) ? cdiv(cdiv(J.H, g) * g * cdiv(J.W, 32), 8 * J.markWords) : 0;
     }
-    case S_COUNT: return J.sparse ? cdiv(J.cw * J.ch, kCountChunk) : 0;
+    case S_COUNT: return J.sparse ? cdiv(J.cw * J.ch, J.countChunk) : 0;
     case S_GATE: return J.useMs ? cdiv(J.cw, 32) * cdiv(J.ch, kGateRows) : 0;
     case S_LGF_DENSE: return (J.guided && J.algo == 4 && !J.lgfRoiOnly) ? cdiv(J.cw, 32) * cdiv(J.ch, 8) : 0;
     case S_HPASS: return (J.hTab && !J.radial && !J.plainFused && (J.kernel != 0 || J.guided)) ? cdiv(J.W, 32) * cdiv(J.ch, 8) : 0;
@@ -974,6 +974,48 @@ static int stageTilesShaped(const FrameJob &J, int s) {
     case S_STORE: return (J.directOutput || J.finalInTransfer || J.blendStores || J.bpStores) ? 0 : cdiv(J.W, 32) * cdiv(J.H, 8);
     }
     return 0;
+}
+
+// Work split of the map and plain stages of one launch. Each of their blocks is
+// a serial walk (rows of a strip, words of a list, rows of a tile), so a launch
+// that leaves most SMs with less than a few blocks takes the length of one
+// walk; shorter walks give it more blocks and cost halo rows. The longest walk
+// whose launch still has kBusyBlocks blocks is taken, else the shortest:
+// one 1080p frame k_tensor 24 -> 20 us (16 rows), k_mark_chroma 17 -> 15 us;
+// one 96x64 frame k_tensor 20 -> 9 us, k_mark_chroma 13 -> 8, k_plain 20 ->
+// 12. 4K frames and batches keep the long walks.
+void shapeJobs(FrameJob *jobs, int n) {
+    constexpr long long kBusyBlocks = 592;         // four per SM
+    auto longest = [&](std::initializer_list<int> sizes, auto blocks) {
+        int size = 0;
+        for (const int s : sizes) {
+            size = s;
+            long long total = 0;
+            for (int f = 0; f < n; ++f)
+                total += blocks(jobs[f], s);
+            if (total >= kBusyBlocks)
+                break;
+        }
+        return size;
+    };
+    const int tensor = longest({kTensorRows, 16, 8}, [](const FrameJob &J, int rows) {
+        return (long long)cdiv(J.sw, kTensorCols * kTensorWarps) * cdiv(J.sh, rows);
+    });
+    const int mark = longest({kMarkWords, 16, 8, 4}, [](const FrameJob &J, int words) {
+        return (long long)cdiv(J.H * cdiv(J.W, 32), 8 * words);
+    });
+    const int count = longest({kCountChunk, 8192, 4096}, [](const FrameJob &J, int bytes) {
+        return (long long)cdiv(J.cw * J.ch, bytes);
+    });
+    const int plain = longest({kPlainRows, 32, 16, 8}, [](const FrameJob &J, int rows) {
+        return (long long)cdiv(J.W, 32) * cdiv(J.H, rows);
+    });
+    for (int f = 0; f < n; ++f) {
+        jobs[f].tensorRows = tensor;
+        jobs[f].markWords = mark;
+        jobs[f].countChunk = count;
+        jobs[f].plainRows = std::min(jobs[f].plainRows, plain);
+    }
 }
 
 void planStages(const std::vector<FrameJob> &jobs, StagePlan &plan, const LaunchConfig *cfg) {

@@ -133,6 +133,10 @@ struct __align__(16) FrameJob {
     int bumpRcpSafe;                   // every guided bump denominator stays below 2^64
     int plainFused;                    // k_plain computes its horizontal rows itself
     int plainRows;                     // output rows per k_plain block
+    // work split of the map stages (shapeJobs)
+    int tensorRows;                    // rows per k_tensor strip
+    int markWords;                     // list words per k_mark_chroma warp
+    int countChunk;                    // chroma mask bytes per k_count block
     int noClampX, noClampY;            // every chroma tap index is in range
     // algo 6 / algo 4 / bm workspaces
     float *aff;                        // cw x ch: float4 (aU aV g rng), float4 (mnU mxU

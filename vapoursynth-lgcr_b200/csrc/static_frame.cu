@@ -238,6 +238,7 @@ extern "C" int lgcr_recon_frame_static(lgcr_recon *h, const lgcr_plane in[3],
     }
     FrameJob job;
     buildJob(t, job);
+    shapeJobs(&job, 1);
     cudaStream_t s = (cudaStream_t)stream;
     e = cudaMemcpyAsync(base, img.bytes.data(), img.bytes.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
