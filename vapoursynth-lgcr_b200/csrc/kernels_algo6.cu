@@ -43,6 +43,7 @@ __device__ __forceinline__ float candidateAt(const FrameJob &J, const WeightView
 }
 
 __global__ void k_yc_h(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int cx, cy;
@@ -87,6 +88,7 @@ __device__ __forceinline__ float ycVertical(const FrameJob &J, const WeightView 
 
 __global__ void __launch_bounds__(256)
 k_yc_tiled(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ float sH1[kYcRows][32];
     __shared__ float sH2[kYcRows][32];
     __shared__ FrameJob sJob;
@@ -212,6 +214,7 @@ __device__ __forceinline__ void affineSample(const FrameJob &J, int x, int y, bo
 // Tiled form (frames without a chroma work list): active samples when sparse.
 __global__ void __launch_bounds__(256, 3)
 k_affine(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ FrameJob sJob;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     stageJob(jobs, f, sJob);
@@ -233,6 +236,7 @@ constexpr int kAffineMaxFrames = 1024;
 
 __global__ void __launch_bounds__(256, 3)
 k_affine_list(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     __shared__ unsigned long long pre[kAffineMaxFrames + 1];
     for (int chunk = 0; chunk < njobs; chunk += kAffineMaxFrames) {
@@ -281,6 +285,7 @@ k_affine_list(const FrameJob *__restrict__ jobs, const int *__restrict__ tileSta
 // plane, src/recon.cpp:1178-1271).
 __global__ void __launch_bounds__(256)
 k_detail_hpass(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, sy;
@@ -306,6 +311,7 @@ k_detail_hpass(LGCR_STAGE_ARGS) {
 
 // detail = Y - plain(D(Y)) on the source luma grid.
 __global__ void k_detail_plain(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -426,6 +432,7 @@ __device__ __forceinline__ double detailVertical(const DetailRows &R, const doub
 
 __global__ void __launch_bounds__(256)
 k_detail_map(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ double sH[kDetailStagedRows][32];
     __shared__ float2 sE[kDetailStagedRows][32];
     __shared__ float sD[kDetailRowsTall + 2][33];
@@ -546,6 +553,7 @@ k_detail_map(LGCR_STAGE_ARGS) {
 // One dyadic pass: x passes (steps 1,2,4..) then y passes; ping-pong
 // between detailTmp and detailTmp2.
 __global__ void k_detail_nyq(LGCR_STAGE_ARGS, int pass) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -570,6 +578,7 @@ __global__ void k_detail_nyq(LGCR_STAGE_ARGS, int pass) {
 }
 
 __global__ void k_detail_resize_h(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -587,6 +596,7 @@ __global__ void k_detail_resize_h(LGCR_STAGE_ARGS) {
 }
 
 __global__ void k_detail_resize_v(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -604,6 +614,7 @@ __global__ void k_detail_resize_v(LGCR_STAGE_ARGS) {
 }
 
 __global__ void k_detail_resize_radial(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int ox, oy;
@@ -702,6 +713,7 @@ __device__ __forceinline__ void transferPixel(const FrameJob &J, int ox, int oy)
     }
 }
 __global__ void k_detail_transfer(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int ox, oy;
@@ -719,6 +731,7 @@ constexpr int kXferMaxFrames = 1024;
 
 __global__ void __launch_bounds__(256)
 k_detail_transfer_list(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     __shared__ unsigned long long pre[kXferMaxFrames + 1];
     for (int chunk = 0; chunk < njobs; chunk += kXferMaxFrames) {
@@ -771,6 +784,7 @@ constexpr int kLgfTile = 1024;               // (bx + 4) * (by + 4) of every blo
 
 __global__ void __launch_bounds__(256)
 k_lgf(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ float sL[kLgfTile], sU[kLgfTile], sV[kLgfTile];
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
@@ -887,6 +901,7 @@ k_lgf(LGCR_STAGE_ARGS) {
 // Mark the 2x2 chroma footprint of output samples whose diagonal routing
 // weight reaches 1e-4.
 __global__ void k_roi(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int ox, oy;
@@ -904,6 +919,7 @@ __global__ void k_roi(LGCR_STAGE_ARGS) {
 }
 
 __global__ void k_blend(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int ox, oy;

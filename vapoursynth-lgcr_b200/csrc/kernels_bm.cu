@@ -70,6 +70,7 @@ __device__ __forceinline__ int anchorCount(const FrameJob &J) { return J.bmAncho
 // One warp per anchor, 8 anchors per block.
 __global__ void __launch_bounds__(256)
 k_bm_group(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ float grp[8][2][64 * kGroup];        // [plane][offset*4 + k]
     __shared__ float costs[8][32];
     __shared__ int cbx[8][32], cby[8][32];
@@ -268,6 +269,7 @@ __device__ __forceinline__ int lowerBound(const int *a, int n, int v) {
 }
 
 __global__ void k_bm_aggregate(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -310,6 +312,7 @@ __global__ void k_bm_aggregate(LGCR_STAGE_ARGS) {
 }
 
 __global__ void k_backproject(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int cx, cy;

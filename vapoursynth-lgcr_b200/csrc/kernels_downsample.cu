@@ -18,6 +18,7 @@
 // All arithmetic is FP32 in the reference's order (the library is compiled
 // without FMA contraction), with its clamped sample reads; quotients are
 // IEEE divisions or refinements equal to them.
+#include "launch.h"
 #include "downsample.h"
 
 namespace lgcr_b200 {
@@ -257,6 +258,7 @@ __device__ __forceinline__ float dsNorm(float sum, float weight, float fallback)
 // Horizontal pass of the base for every source row.
 template <int KIND>
 __global__ void __launch_bounds__(128) k_ds_rows(DownsampleJob J) {
+    gridDependency();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= J.cw)
         return;
@@ -274,6 +276,7 @@ __global__ void __launch_bounds__(128) k_ds_rows(DownsampleJob J) {
 // Vertical pass, then (GUIDED) the guided correction or the candidates.
 template <int KIND, bool GUIDED>
 __global__ void __launch_bounds__(256) k_ds_pixel(DownsampleJob J) {
+    gridDependency();
     __shared__ float sY[GUIDED ? kDsTw * kDsTh : 1], sU[GUIDED ? kDsTw * kDsTh : 1],
         sV[GUIDED ? kDsTw * kDsTh : 1];
     __shared__ float sW[GUIDED ? kDsMaxTaps * kDsSlots : 1];
@@ -380,6 +383,7 @@ constexpr int kDsSw = kDsBx + 2, kDsSh = kDsBy + 2;
 
 template <int KIND>
 __global__ void __launch_bounds__(256) k_ds_score(DownsampleJob J) {
+    gridDependency();
     __shared__ float2 sC[4][kDsSh][kDsSw];             // blended (U, V) of each candidate
     const int bx0 = blockIdx.x * kDsBx, by0 = blockIdx.y * kDsBy;
     const int x = bx0 + threadIdx.x, y = by0 + threadIdx.y;
@@ -451,14 +455,14 @@ __global__ void __launch_bounds__(256) k_ds_score(DownsampleJob J) {
 
 template <int KIND>
 cudaError_t launchKind(const DownsampleJob &J, cudaStream_t s) {
-    k_ds_rows<KIND><<<dim3((J.cw + 127) / 128, J.H), 128, 0, s>>>(J);
+    launchAfter(k_ds_rows<KIND>, dim3((J.cw + 127) / 128, J.H), 128, 0, s, J);
     const dim3 grid((J.cw + kDsBx - 1) / kDsBx, (J.ch + kDsBy - 1) / kDsBy), block(kDsBx, kDsBy);
     if (J.strength == 0.0f) {
-        k_ds_pixel<KIND, false><<<grid, block, 0, s>>>(J);
+        launchAfter(k_ds_pixel<KIND, false>, grid, block, 0, s, J);
     } else {
-        k_ds_pixel<KIND, true><<<grid, block, 0, s>>>(J);
+        launchAfter(k_ds_pixel<KIND, true>, grid, block, 0, s, J);
         if (J.quality == 2)
-            k_ds_score<KIND><<<grid, block, 0, s>>>(J);
+            launchAfter(k_ds_score<KIND>, grid, block, 0, s, J);
     }
     return cudaGetLastError();
 }

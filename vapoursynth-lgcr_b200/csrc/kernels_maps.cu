@@ -241,6 +241,7 @@ __device__ __forceinline__ void convertChroma(const FrameJob &J, int cy, int xb,
 
 __global__ void __launch_bounds__(kConvertWarps * 32, 3)
 k_convert(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ FrameJob sJob;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     stageJob(jobs, f, sJob);
@@ -301,6 +302,7 @@ __device__ __forceinline__ void sobel(const Tri &t, const Tri &c, const Tri &b, 
 
 __global__ void __launch_bounds__(kTensorWarps * 32)
 k_tensor(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     const int tile = blockIdx.x - tileStart[f];
@@ -396,6 +398,7 @@ __device__ __forceinline__ uint32_t packNibble(uint32_t fourBytes) {
 
 __global__ void __launch_bounds__(128)
 k_dilate_h(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ uint32_t words[kDilMaxWords + 2 * kDilPadWords];
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
@@ -445,6 +448,7 @@ k_dilate_h(LGCR_STAGE_ARGS) {
 // Also counts the set mask samples (one atomic per block).
 __global__ void __launch_bounds__(256)
 k_dilate_v(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ unsigned warpSum[8];
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
@@ -518,6 +522,7 @@ __device__ __forceinline__ uint32_t activeWord(const FrameJob &J, int kw, int oy
 
 __global__ void __launch_bounds__(256)
 k_mark_chroma(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ unsigned warpCount[8];
     __shared__ unsigned long long blockBase;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
@@ -588,6 +593,7 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
 // raster order at the block's range.
 __global__ void __launch_bounds__(256)
 k_count(LGCR_STAGE_ARGS) {
+    gridDependency();
     __shared__ unsigned warpSum[8];
     __shared__ unsigned long long blockBase;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
@@ -738,6 +744,7 @@ __device__ __forceinline__ float gateAt(const GateTile &T, int x, int y, int x0,
 
 __global__ void __launch_bounds__(GT_X * 8)
 k_gate(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     constexpr int SW = GW + 2, SH = GHh + 2;     // lc, U, V with the Sobel ring
     __shared__ float src[3][SH][SW];
     __shared__ GateTile T;

@@ -131,6 +131,7 @@ __device__ __forceinline__ void storeEntry(const FrameJob &J, int ox, int sy, co
 // rows in shared memory).
 __global__ void __launch_bounds__(256)
 k_hpass(LGCR_STAGE_ARGS) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int ox, sy;
@@ -680,6 +681,7 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
 
 __global__ void __launch_bounds__(256, 4)
 k_plain(LGCR_STAGE_ARGS) {
+    gridDependency();
     plainStage<false>(jobs, tileStart, njobs);
 }
 
@@ -687,6 +689,7 @@ k_plain(LGCR_STAGE_ARGS) {
 // every output pixel): returns at once for frames the guided pass covers
 __global__ void __launch_bounds__(256, 4)
 k_plain_all(LGCR_STAGE_ARGS) {
+    gridDependency();
     plainStage<true>(jobs, tileStart, njobs);
 }
 
@@ -1534,18 +1537,21 @@ __device__ __forceinline__ void guidedGrid(const FrameJob *__restrict__ jobs, in
 // autotuner picks.
 __global__ void __launch_bounds__(256, 2)
 k_guided(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<2, false, false>(jobs, njobs);
 }
 
 __global__ void __launch_bounds__(256, 3)
 k_guided3(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<3, false, false>(jobs, njobs);
 }
 
 __global__ void __launch_bounds__(256, 2)
 k_guided_staged(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<2, true, false>(jobs, njobs);
 }
@@ -1553,18 +1559,21 @@ k_guided_staged(const FrameJob *__restrict__ jobs, const int *__restrict__ tileS
 // the same three for batches with jinc selector frames
 __global__ void __launch_bounds__(256, 2)
 k_guided_r(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<2, false, true>(jobs, njobs);
 }
 
 __global__ void __launch_bounds__(256, 3)
 k_guided3_r(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<3, false, true>(jobs, njobs);
 }
 
 __global__ void __launch_bounds__(256, 2)
 k_guided_staged_r(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<2, true, true>(jobs, njobs);
 }
@@ -1572,18 +1581,21 @@ k_guided_staged_r(const FrameJob *__restrict__ jobs, const int *__restrict__ til
 // and for launches of jinc selector frames only
 __global__ void __launch_bounds__(256, 2)
 k_guided_o(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<2, false, true, true>(jobs, njobs);
 }
 
 __global__ void __launch_bounds__(256, 3)
 k_guided3_o(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<3, false, true, true>(jobs, njobs);
 }
 
 __global__ void __launch_bounds__(256, 2)
 k_guided_staged_o(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     (void)tileStart;
     guidedGrid<2, true, true, true>(jobs, njobs);
 }
@@ -1591,6 +1603,7 @@ k_guided_staged_o(const FrameJob *__restrict__ jobs, const int *__restrict__ til
 // Float output planes -> typed output (output conversion stage).
 __global__ void k_store_chroma(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart,
                                int njobs) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int ox, oy;
@@ -1608,6 +1621,7 @@ __global__ void k_store_chroma(const FrameJob *__restrict__ jobs, const int *__r
 // ---------------------------------------------------------------------------
 __global__ void k_luma_h(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart,
                          int njobs) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -1626,6 +1640,7 @@ __global__ void k_luma_h(const FrameJob *__restrict__ jobs, const int *__restric
 
 __global__ void k_luma_v(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart,
                          int njobs) {
+    gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
     int x, y;
@@ -1675,6 +1690,7 @@ __device__ __forceinline__ void radialTabled(const double *__restrict__ w, const
 
 __global__ void __launch_bounds__(256)
 k_luma_radial(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+    gridDependency();
     __shared__ double sY[kRadialTileMax];
     __shared__ double sW[kRadialWeightsMax];
     __shared__ float sDx[kRadialBx][kRadialMaxSup], sDy[kRadialBy][kRadialMaxSup];

@@ -26,6 +26,7 @@
 // One 1080p 4:2:0 10-bit frame with two neighbours, tsearch 6: matching
 // 124 -> 93 us, consistency 119 -> 32 us.
 #include "temporal.cuh"
+#include "launch.h"
 #include "trecon.h"
 
 #include <algorithm>
@@ -79,6 +80,7 @@ __device__ __forceinline__ bool rawFloat4(const void *base, long long pitch, int
 // for three 1080p frames).
 template <int KIND>
 __global__ void __launch_bounds__(256) k_trecon_convert(const TReconPrep P) {
+    gridDependency();
     const int frame = blockIdx.y / 3, plane = blockIdx.y % 3;
     const int w = plane ? P.cw : P.sw, h = plane ? P.ch : P.sh;
     const double off = plane ? P.cOffset : 0.0;
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(256) k_trecon_convert(const TReconPrep P) {
 
 // blockIdx.y: neighbour - 1; a warp takes row segments of 32 samples
 __global__ void __launch_bounds__(256) k_trecon_lc(const TReconPrep P) {
+    gridDependency();
     const int k = 1 + blockIdx.y;
     const float *Y = P.f[k][0];
     float *lc = P.lc[k];
@@ -138,6 +141,7 @@ __host__ __device__ __forceinline__ void matchWindow(int search, int &extent, in
 // blockIdx.x: block index, blockIdx.y: neighbour - 1
 template <bool STAGED>
 __global__ void __launch_bounds__(kMatchThreads) k_block_match(const TReconPrep P) {
+    gridDependency();
     extern __shared__ float win[];
     __shared__ __align__(16) float cur[kTReconBlock / 2][kTReconBlock / 2];
     __shared__ unsigned long long best[kMatchThreads / 32];
@@ -253,6 +257,7 @@ constexpr int kConsistMax = 256;            // 16 x 16 deltas at most (4:4:4)
 
 // Blocks of the smallest multiple of 32 threads that gives every delta one.
 __global__ void __launch_bounds__(kConsistMax) k_chroma_consist(const TReconPrep P) {
+    gridDependency();
     __shared__ __align__(16) unsigned d[kConsistMax];
     __shared__ unsigned middle[2];
     const int k = 1 + blockIdx.y;
@@ -311,6 +316,7 @@ __global__ void __launch_bounds__(kConsistMax) k_chroma_consist(const TReconPrep
 
 __global__ void k_trecon_lanczos(double *tabX, double *tabY, double rw, double rh, float invWx, float invWy,
                                  double support) {
+    gridDependency();
     const int i = threadIdx.x;
     const float d = (float)i / (float)kTLanSteps;
     tabX[i] = temporalLanczos(d, rw, invWx, support);
@@ -320,14 +326,14 @@ __global__ void k_trecon_lanczos(double *tabX, double *tabY, double rw, double r
 template <int KIND>
 void convertKind(const TReconPrep &P, cudaStream_t s) {
     const int segs = (P.sw + 127) / 128 * P.sh;
-    k_trecon_convert<KIND><<<dim3(std::min((segs + 7) / 8, 1184), 3 * P.frames), 256, 0, s>>>(P);
+    launchAfter(k_trecon_convert<KIND>, dim3(std::min((segs + 7) / 8, 1184), 3 * P.frames), 256, 0, s, P);
 }
 
 } // namespace
 
 void launchTReconLanczos(double *tabX, double *tabY, double rw, double rh, float invWx, float invWy,
                          double support, cudaStream_t s) {
-    k_trecon_lanczos<<<1, kTLanEntries, 0, s>>>(tabX, tabY, rw, rh, invWx, invWy, support);
+    launchAfter(k_trecon_lanczos, 1, kTLanEntries, 0, s, tabX, tabY, rw, rh, invWx, invWy, support);
 }
 
 int launchTReconPrep(const TReconPrep &P, cudaStream_t s) {
@@ -340,22 +346,22 @@ int launchTReconPrep(const TReconPrep &P, cudaStream_t s) {
     default: convertKind<kF32>(P, s); break;
     }
     const int segs = (P.cw + 31) / 32 * P.ch;
-    k_trecon_lc<<<dim3(std::min((segs + 7) / 8, 1184), nbrs), 256, 0, s>>>(P);
+    launchAfter(k_trecon_lc, dim3(std::min((segs + 7) / 8, 1184), nbrs), 256, 0, s, P);
     int extent, pitch;
     matchWindow(P.search, extent, pitch);
     const int window = extent * pitch;
     const int cands = (2 * P.search + 1) * (2 * P.search + 1);
     const int threads = std::min(kMatchThreads, (cands + 31) / 32 * 32);
     if (window <= kMatchWindowMax)
-        k_block_match<true><<<dim3(P.bw * P.bh, nbrs), threads, window * sizeof(float), s>>>(P);
+        launchAfter(k_block_match<true>, dim3(P.bw * P.bh, nbrs), threads, window * sizeof(float), s, P);
     else
-        k_block_match<false><<<dim3(P.bw * P.bh, nbrs), threads, 0, s>>>(P);
+        launchAfter(k_block_match<false>, dim3(P.bw * P.bh, nbrs), threads, 0, s, P);
     // chroma samples of a luma block, at most one more per axis than its share
     const int perX = std::min(kTReconBlock, (int)(kTReconBlock / P.rw) + 2);
     const int perY = std::min(kTReconBlock, (int)(kTReconBlock / P.rh) + 2);
     const bool whole = P.rw == 2.0 && P.rh == 2.0;
     const int deltas = whole ? kTReconBlock * kTReconBlock / 4 : perX * perY;
-    k_chroma_consist<<<dim3(P.bw * P.bh, nbrs), (deltas + 31) / 32 * 32, 0, s>>>(P);
+    launchAfter(k_chroma_consist, dim3(P.bw * P.bh, nbrs), (deltas + 31) / 32 * 32, 0, s, P);
     return cudaGetLastError() == cudaSuccess ? 4 : -1;
 }
 

@@ -4,6 +4,7 @@
 // with one launch per stage covering every frame of a batch.
 #include "impl.h"
 #include "kernels.cuh"
+#include "launch.h"
 
 #include <algorithm>
 #include <cmath>
@@ -1049,7 +1050,7 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
             return;
         if (stageTunable(s))
             block = dim3(plan.cfg.shapeX[s], plan.cfg.shapeY[s]);
-        kernel<<<plan.totals[s], block, smem, stream>>>(dJobs, pre(s), n);
+        launchAfter(kernel, dim3(plan.totals[s]), block, smem, stream, dJobs, pre(s), n);
         ++launches;
     };
     go(S_CONVERT, k_convert, dim3(kConvertWarps * 32));
@@ -1112,7 +1113,7 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, 256, dyn);
             grid = std::max(1, sms * std::max(1, perSm));
         }
-        kern<<<grid, 256, dyn, stream>>>(dJobs, pre(S_GUIDED), n);
+        launchAfter(kern, dim3(grid), dim3(256), dyn, stream, dJobs, pre(S_GUIDED), n);
         ++launches;
     }
     go(S_YC, k_yc_h, b32x8);
@@ -1128,7 +1129,7 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_affine_list, 256, 0);
             gridBlocks = std::max(1, sms * std::max(1, perSm));
         }
-        k_affine_list<<<gridBlocks, 256, 0, stream>>>(dJobs, pre(S_AFFINE_LIST), n);
+        launchAfter(k_affine_list, dim3(gridBlocks), dim3(256), 0, stream, dJobs, pre(S_AFFINE_LIST), n);
         ++launches;
     }
     go(S_DET_HPASS, k_detail_hpass, b32x8);
@@ -1138,7 +1139,7 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
         const int s = S_NYQ0 + pass;
         if (plan.totals[s] == 0)
             continue;
-        k_detail_nyq<<<plan.totals[s], b32x8, 0, stream>>>(dJobs, pre(s), n, pass);
+        launchAfter(k_detail_nyq, dim3(plan.totals[s]), b32x8, 0, stream, dJobs, pre(s), n, pass);
         ++launches;
     }
     go(S_DET_RH, k_detail_resize_h, b32x8);
@@ -1155,7 +1156,7 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_detail_transfer_list, 256, 0);
             gridBlocks = std::max(1, sms * std::max(1, perSm));
         }
-        k_detail_transfer_list<<<gridBlocks, 256, 0, stream>>>(dJobs, pre(S_DET_XFER_LIST), n);
+        launchAfter(k_detail_transfer_list, dim3(gridBlocks), dim3(256), 0, stream, dJobs, pre(S_DET_XFER_LIST), n);
         ++launches;
     }
     go(S_ROI, k_roi, b32x8);

@@ -277,6 +277,14 @@ __device__ __forceinline__ uint32_t maskAt(const FrameJob &J, int x, int y) {
     return (__ldg(J.mask + (size_t)y * J.maskWords + (x >> 5)) >> (x & 31)) & 1u;
 }
 
+// First statement of every kernel launched with launchAfter (launch.h), which
+// may be set up while the one before it ends; this waits until that one has completed and its writes are
+// visible. No kernel signals completion early, so blocks start when all blocks
+// of the previous kernel have exited.
+__device__ __forceinline__ void gridDependency() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Shared-memory copy of one frame's job for the whole block. Kernels that
 // read FrameJob fields inside loops with global stores read them from this
 // copy, so the fields are not reloaded from global memory after each store.
