@@ -6,6 +6,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <string>
+#include <string>
 #include <unordered_map>
 
 namespace lgcr_b200 {
@@ -292,6 +294,116 @@ void rescueFactors(const ChromaAxis &a, std::vector<float> &mx, std::vector<floa
         }
         mx[i] = m;
         ss[i] = q;
+    }
+}
+
+PairAxis buildPairAxis(const ChromaAxis &a, int chromaN, float r) {
+    PairAxis t;
+    const int n = (a.n + 1) / 2;
+    std::vector<int> lo(n), hi(n);
+    int widest = kPairMinSup;
+    for (int p = 0; p < n; ++p) {
+        lo[p] = chromaN;
+        hi[p] = -1;
+        for (int x = 2 * p; x < std::min(2 * p + 2, a.n); ++x)
+            for (int j = 0; j < a.sup; ++j)
+                if (a.am[size_t(x) * a.sup + j]) {
+                    lo[p] = std::min(lo[p], a.start[x] + j);
+                    hi[p] = std::max(hi[p], a.start[x] + j);
+                }
+        if (hi[p] < 0 || hi[p] >= chromaN)
+            return t;                             // a column without taps, or taps past the plane
+        widest = std::max(widest, hi[p] - lo[p] + 1);
+    }
+    if (widest > kPairMaxSup || widest > chromaN)
+        return t;
+    t.n = n;
+    t.sup = widest;
+    t.start.resize(n);
+    t.kind.resize(n);
+    t.bits.assign(n, 0u);
+    t.first.assign(size_t(n) * 2, 0);
+    const size_t per = size_t(widest) * 4;
+    std::vector<float> row(per);
+    std::unordered_map<std::string, int> kinds;
+    for (int p = 0; p < n; ++p) {
+        const int s = std::clamp(lo[p], 0, chromaN - widest);
+        t.start[p] = s;
+        std::fill(row.begin(), row.end(), 0.0f);
+        for (int q = 0; q < 2 && 2 * p + q < a.n; ++q) {
+            const int x = 2 * p + q;
+            t.first[size_t(p) * 2 + q] = a.start[x] - s;
+            for (int j = 0; j < a.sup; ++j) {
+                if (!a.am[size_t(x) * a.sup + j])
+                    continue;
+                const int i = a.start[x] + j - s;
+                t.bits[p] |= 1u << (i + 16 * q);
+                row[size_t(i) * 4 + q] = a.w[size_t(x) * a.sup + j];
+            }
+        }
+        for (int q = 0; q < 2; ++q)
+            for (int i = 0; i < widest; ++i)
+                row[size_t(i) * 4 + 2 + q] = (float(s + i) - a.pos[std::min(2 * p + q, a.n - 1)]) * r;
+        const std::string key(reinterpret_cast<const char *>(row.data()), per * sizeof(float));
+        const auto [it, fresh] = kinds.emplace(key, int(kinds.size()));
+        if (fresh)
+            t.tab.insert(t.tab.end(), row.begin(), row.end());
+        t.kind[p] = it->second;
+    }
+    return t;
+}
+
+PairRadial buildPairRadial(const RadialTable &t, const PairAxis &p, int outN) {
+    PairRadial r;
+    if (!t.valid || p.sup == 0)
+        return r;
+    struct Kind { int px[2], first[2]; };
+    std::vector<Kind> kinds;
+    r.phase.resize(p.n);
+    for (int i = 0; i < p.n; ++i) {
+        const int x1 = std::min(2 * i + 1, outN - 1);
+        Kind k{{t.xPhase[2 * i], t.xPhase[x1]}, {p.first[size_t(i) * 2], p.first[size_t(i) * 2 + 1]}};
+        if (x1 == 2 * i)
+            k.first[1] = k.first[0];              // an odd width's last column
+        size_t at = 0;
+        while (at < kinds.size() && std::memcmp(&kinds[at], &k, sizeof(k)) != 0)
+            ++at;
+        if (at == kinds.size()) {
+            if ((kinds.size() + 1) * t.phaseCountY > 1024)
+                return r;
+            kinds.push_back(k);
+        }
+        r.phase[i] = uint16_t(at);
+    }
+    r.phasePairs = int(kinds.size());
+    const size_t per = size_t(t.supportY) * p.sup * 2;
+    r.w.assign(per * r.phasePairs * t.phaseCountY, 0.0f);
+    for (int py = 0; py < t.phaseCountY; ++py)
+        for (int k = 0; k < r.phasePairs; ++k)
+            for (int q = 0; q < 2; ++q) {
+                const float *src = t.weights.data() +
+                    (size_t(py) * t.phaseCountX + kinds[k].px[q]) * t.supportX * t.supportY;
+                float *dst = r.w.data() + per * (size_t(py) * r.phasePairs + k);
+                for (int j = 0; j < t.supportY; ++j)
+                    for (int i = 0; i < t.supportX; ++i) {
+                        const int c = i + kinds[k].first[q];
+                        if (c >= 0 && c < p.sup)  // taps outside the window are inactive
+                            dst[(size_t(j) * p.sup + c) * 2 + q] = src[size_t(j) * t.supportX + i];
+                    }
+            }
+    r.valid = true;
+    return r;
+}
+
+void phaseTables(const ChromaAxis &a, int chromaN, std::vector<float> &gate,
+                 std::vector<int> &nearest) {
+    gate.resize(a.n);
+    nearest.resize(a.n);
+    for (int i = 0; i < a.n; ++i) {
+        const float f = a.pos[i] - std::floor(a.pos[i]);
+        const float other = 1.0f - f;
+        gate[i] = 1.0f - 2.0f * (other < f ? other : f);
+        nearest[i] = std::clamp(int(std::lround(a.pos[i])), 0, chromaN - 1);
     }
 }
 

@@ -82,6 +82,42 @@ RadialTable buildRadialTable(const KernelSpec &k, const ChromaAxis &ax, const Ch
 // factors), in float and in tap order as the guided pass evaluates them.
 void rescueFactors(const ChromaAxis &a, std::vector<float> &mx, std::vector<float> &ss);
 
+// Pairs of output columns (2p, 2p + 1) of a chroma axis on one common window
+// of `sup` samples: the guided pass evaluates both pixels of a pair from the
+// same loaded samples. Empty (sup 0) when some pair's active taps span more
+// than kPairMaxSup samples or the plane is narrower than the window.
+constexpr int kPairMinSup = 4, kPairMaxSup = 9;
+struct PairAxis {
+    int n = 0, sup = 0;
+    std::vector<int> start;      // first sample of the common window
+    // per pair the row of `tab`, the distinct pairs' taps: [kind][sup][4] with
+    // both columns' weights (zero at inactive taps) and then both columns' tap
+    // distances (tap - position) * r in float. Away from the frame's sides a
+    // same-size frame has one kind.
+    std::vector<int> kind;
+    std::vector<float> tab;
+    std::vector<uint32_t> bits;  // active taps: low half column 2p, high half column 2p + 1
+    std::vector<int> first;      // n * 2: tap of the common window that is tap 0 of the column
+};
+PairAxis buildPairAxis(const ChromaAxis &a, int chromaN, float r);
+
+// Jinc weights of both columns of a pair on the common window, per (row
+// phase, phase pair): phase pairs are the distinct (column phases, tap
+// offsets) of the pairs. Not valid when the radial table is not, or with more
+// than 1024 (row phase, phase pair) combinations.
+struct PairRadial {
+    bool valid = false;
+    int phasePairs = 0;
+    std::vector<uint16_t> phase;     // per pair
+    std::vector<float> w;            // [row phase][phase pair][row][column of the window][2]
+};
+PairRadial buildPairRadial(const RadialTable &t, const PairAxis &p, int outN);
+
+// Per index: the phase gate factor 1 - 2 * min(f, 1 - f) of the position's
+// fraction f, and the nearest sample (round half away from zero, clamped).
+void phaseTables(const ChromaAxis &a, int chromaN, std::vector<float> &gate,
+                 std::vector<int> &nearest);
+
 // Footprint extents of each chroma sample on the luma grid.
 void lcExtents(int lumaN, int chromaN, double r, double shift,
                std::vector<int> &begin, std::vector<int> &end);

@@ -58,6 +58,15 @@ struct DeviceTables {
     DeviceArena arena;
     AxisView ax{}, ay{};
     RadialView rad{};
+    // guided pass by column pairs (0: this table set has none)
+    int pairSup = 0, pairPhases = 0;
+    const int *pairStart = nullptr;
+    const uint32_t *pairBits = nullptr;
+    const int *pairKind = nullptr;
+    const float *pairTab = nullptr;
+    const uint16_t *pairPhase = nullptr;
+    const float *pairRad = nullptr;
+    const double *pairRadD = nullptr, *radSums = nullptr;
     WeightView lumaH{}, lumaV{};
     const int *lcXb = nullptr, *lcXe = nullptr, *lcYb = nullptr, *lcYe = nullptr;
     // algo 6
@@ -96,6 +105,7 @@ struct Workspace {
     double *uvd = nullptr;
     float *hTab = nullptr;
     float *wExt = nullptr;              // W x H float4 hull plane, then W x H float2 luma plane
+    float *context = nullptr;           // guided pixel contexts (in hTab's region where that is free)
     uint32_t *actList = nullptr;
     uint32_t *chromaList = nullptr;
     float *aff = nullptr, *yc1 = nullptr, *yc2 = nullptr, *ycTmp = nullptr;

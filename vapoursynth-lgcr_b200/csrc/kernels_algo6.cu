@@ -649,8 +649,8 @@ __global__ void k_detail_resize_radial(LGCR_STAGE_ARGS) {
 __device__ __forceinline__ bool activeOut(const FrameJob &J, int ox, int oy) {
     if (!J.sparse)
         return true;
-    const int mx = J.sameSize ? ox : min(J.sw - 1, (int)((long long)ox * J.sw / J.W));
-    const int my = J.sameSize ? oy : min(J.sh - 1, (int)((long long)oy * J.sh / J.H));
+    const int mx = J.sameSize ? ox : min(J.sw - 1, maskIndex(ox, J.sw, J.W));
+    const int my = J.sameSize ? oy : min(J.sh - 1, maskIndex(oy, J.sh, J.H));
     return maskAt(J, mx, my) != 0;
 }
 
@@ -782,6 +782,11 @@ __device__ __forceinline__ float pointLuma(const FrameJob &J, int x, int y) {
 // an ROI sample only store the maps' zeros.
 constexpr int kLgfTile = 1024;               // (bx + 4) * (by + 4) of every block shape used
 
+__device__ __forceinline__ void storeLgf(const FrameJob &J, size_t o, float4 ab, float2 conf) {
+    reinterpret_cast<float4 *>(J.lgf)[o] = ab;
+    reinterpret_cast<float2 *>(J.lgf + 4 * (size_t)J.cw * J.ch)[o] = conf;
+}
+
 __global__ void __launch_bounds__(256)
 k_lgf(LGCR_STAGE_ARGS) {
     gridDependency();
@@ -803,12 +808,8 @@ k_lgf(LGCR_STAGE_ARGS) {
         // outside the ROI the maps hold zeros (buildLGFMaps fills them before
         // the ROI pass, recon.cpp:1541-1548); the blend reads them wherever
         // w2 or w3 reaches 1e-4, which includes samples outside the ROI
-        if (inside) {
-            const size_t C = (size_t)w * h;
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                J.lgf[k * C + o] = 0.0f;
-        }
+        if (inside)
+            storeLgf(J, o, make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float2(0.0f, 0.0f));
         return;
     }
     if (staged) {
@@ -823,10 +824,7 @@ k_lgf(LGCR_STAGE_ARGS) {
     if (!inside)
         return;
     if (!work) {
-        const size_t C = (size_t)w * h;
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-            J.lgf[k * C + o] = 0.0f;
+        storeLgf(J, o, make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float2(0.0f, 0.0f));
         return;
     }
     const int top = max(0, y - 2), bottom = min(h - 1, y + 2);
@@ -856,12 +854,8 @@ k_lgf(LGCR_STAGE_ARGS) {
     const double meanU = s[2] / n, meanV = s[4] / n;
     const double slopeU = (s[3] / n - meanY * meanU) / (var + eps);
     const double slopeV = (s[5] / n - meanY * meanV) / (var + eps);
-    const size_t C = (size_t)w * h;
-    float *L = J.lgf;
-    L[0 * C + o] = (float)slopeU;
-    L[1 * C + o] = (float)(meanU - slopeU * meanY);
-    L[3 * C + o] = (float)slopeV;
-    L[4 * C + o] = (float)(meanV - slopeV * meanY);
+    const float4 ab = make_float4((float)slopeU, (float)(meanU - slopeU * meanY), (float)slopeV,
+                                  (float)(meanV - slopeV * meanY));
     const float base = (float)(var / (var + eps));
     float confU = base, confV = base;
     if (J.cedge) {
@@ -894,8 +888,7 @@ k_lgf(LGCR_STAGE_ARGS) {
         confU *= fm;
         confV *= fm;
     }
-    L[2 * C + o] = confU;
-    L[5 * C + o] = confV;
+    storeLgf(J, o, ab, make_float2(confU, confV));
 }
 
 // Mark the 2x2 chroma footprint of output samples whose diagonal routing
@@ -945,8 +938,6 @@ __global__ void k_blend(LGCR_STAGE_ARGS) {
     const float lam = J.strength4;
     const bool compressed = J.sparse &&
         (unsigned long long)J.counters[kCntActiveOutput] * 2ull < (unsigned long long)J.W * J.H;
-    const int cw = J.cw, ch = J.ch;
-    const size_t C = (size_t)cw * ch;
     const int cx = __ldg(J.ax.cbI0 + ox), cy = __ldg(J.ay.cbI0 + oy);
     const float cxf = __ldg(J.ax.cbF + ox), cyf = __ldg(J.ay.cbF + oy);
     const float plainU = J.oU[o], plainV = J.oV[o];
@@ -957,12 +948,8 @@ __global__ void k_blend(LGCR_STAGE_ARGS) {
         if (w3 != 0.0f) {
             const float luma = bilinearFast(J.Y, J.sw, J.sh, __ldg(J.ax.lbI0 + ox), __ldg(J.ax.lbF + ox),
                                             __ldg(J.ay.lbI0 + oy), __ldg(J.ay.lbF + oy));
-            const float au = bilinearFast(J.lgf + 0 * C, cw, ch, cx, cxf, cy, cyf);
-            const float bu = bilinearFast(J.lgf + 1 * C, cw, ch, cx, cxf, cy, cyf);
-            const float cu = bilinearFast(J.lgf + 2 * C, cw, ch, cx, cxf, cy, cyf);
-            const float av = bilinearFast(J.lgf + 3 * C, cw, ch, cx, cxf, cy, cyf);
-            const float bv = bilinearFast(J.lgf + 4 * C, cw, ch, cx, cxf, cy, cyf);
-            const float cv = bilinearFast(J.lgf + 5 * C, cw, ch, cx, cxf, cy, cyf);
+            const LgfSample m = lgfAt(J, cx, cxf, cy, cyf);
+            const float au = m.ab.x, bu = m.ab.y, av = m.ab.z, bv = m.ab.w, cu = m.conf.x, cv = m.conf.y;
             valueU += w3 * cu * (au * luma + bu - plainU);
             valueV += w3 * cv * (av * luma + bv - plainV);
         }
@@ -978,12 +965,8 @@ __global__ void k_blend(LGCR_STAGE_ARGS) {
     }
     const float L0 = bilinearFast(J.Y, J.sw, J.sh, __ldg(J.ax.lbI0 + ox), __ldg(J.ax.lbF + ox),
                                   __ldg(J.ay.lbI0 + oy), __ldg(J.ay.lbF + oy));
-    const float au = bilinearFast(J.lgf + 0 * C, cw, ch, cx, cxf, cy, cyf);
-    const float bu = bilinearFast(J.lgf + 1 * C, cw, ch, cx, cxf, cy, cyf);
-    const float cu = bilinearFast(J.lgf + 2 * C, cw, ch, cx, cxf, cy, cyf);
-    const float av = bilinearFast(J.lgf + 3 * C, cw, ch, cx, cxf, cy, cyf);
-    const float bv = bilinearFast(J.lgf + 4 * C, cw, ch, cx, cxf, cy, cyf);
-    const float cv = bilinearFast(J.lgf + 5 * C, cw, ch, cx, cxf, cy, cyf);
+    const LgfSample m = lgfAt(J, cx, cxf, cy, cyf);
+    const float au = m.ab.x, bu = m.ab.y, av = m.ab.z, bv = m.ab.w, cu = m.conf.x, cv = m.conf.y;
     finish(plainU + (w2v * (J.gU[o] - plainU) + w3v * cu * (au * L0 + bu - plainU)),
            plainV + (w2v * (J.gV[o] - plainV) + w3v * cv * (av * L0 + bv - plainV)));
 }

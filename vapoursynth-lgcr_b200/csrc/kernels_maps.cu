@@ -511,10 +511,10 @@ __device__ __forceinline__ uint32_t activeWord(const FrameJob &J, int kw, int oy
         return valid;
     if (J.sameSize)
         return __ldg(J.mask + (size_t)oy * J.maskWords + kw) & valid;
-    const int my = min(J.sh - 1, (int)((long long)oy * J.sh / J.H));
+    const int my = min(J.sh - 1, maskIndex(oy, J.sh, J.H));
     uint32_t bits = 0;
     for (int i = 0; i < n; ++i) {
-        const int mx = min(J.sw - 1, (int)((long long)(x0 + i) * J.sw / J.W));
+        const int mx = min(J.sw - 1, maskIndex(x0 + i, J.sw, J.W));
         bits |= maskAt(J, mx, my) << i;
     }
     return bits;
@@ -523,7 +523,7 @@ __device__ __forceinline__ uint32_t activeWord(const FrameJob &J, int kw, int oy
 __global__ void __launch_bounds__(256)
 k_mark_chroma(LGCR_STAGE_ARGS) {
     gridDependency();
-    __shared__ unsigned warpCount[8];
+    __shared__ unsigned warpCount[8], warpPixels[8];
     __shared__ unsigned long long blockBase;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
@@ -539,23 +539,35 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
     markWord(wordBase + lane, ow, J.listGroup, myOy, myKw);
     if (lane < per && myOy < J.H)
         myBits = activeWord(J, myKw, myOy);
-    const unsigned cnt = __popc(myBits);
+    // list entries of the word: pixels, or column pairs with an active pixel
+    const bool pairs = J.pairSup > 0;
+    const unsigned pixels = __reduce_add_sync(0xffffffffu, (unsigned)__popc(myBits));
+    const unsigned cnt = __popc(pairs ? (myBits | myBits >> 1) & 0x55555555u : myBits);
     unsigned incl = cnt;
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned n = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += n;
     }
-    if (lane == 31)
+    if (lane == 31) {
         warpCount[warp] = incl;
+        warpPixels[warp] = pixels;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned total = 0;
+        unsigned total = 0, all = 0;
         for (int i = 0; i < 8; ++i) {
             const unsigned c = warpCount[i];
             warpCount[i] = total;
             total += c;
+            all += warpPixels[i];
         }
-        blockBase = total ? atomicAdd(J.counters + kCntActiveOutput, (unsigned long long)total) : 0ull;
+        blockBase = 0ull;
+        if (total) {
+            blockBase = atomicAdd(J.counters + (pairs ? kCntPairs : kCntActiveOutput),
+                                  (unsigned long long)total);
+            if (pairs)
+                atomicAdd(J.counters + kCntActiveOutput, (unsigned long long)all);
+        }
     }
     __syncthreads();
     const unsigned long long warpBase = blockBase + warpCount[warp];
@@ -569,9 +581,15 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
             continue;                                      // warp-uniform
         const int oy = __shfl_sync(0xffffffffu, myOy, i);
         const int kw = __shfl_sync(0xffffffffu, myKw, i);
+        const int ox = kw * 32 + lane;
+        if (pairs) {
+            const uint32_t both = (bits >> (lane & ~1)) & 3u, pb = (bits | bits >> 1) & 0x55555555u;
+            if (!(lane & 1) && both)
+                J.actList[warpBase + offs + __popc(pb & below)] =
+                    ((uint32_t)oy << 16) | (uint32_t)ox | (both == 3u ? 0u : 1u);
+        }
         if (!((bits >> lane) & 1u))
             continue;
-        const int ox = kw * 32 + lane;
         if (J.sparse) {
             const int cy0 = __ldg(J.ay.cbI0 + oy);
             const int cy1 = min(cy0 + 1, J.ch - 1);
@@ -582,7 +600,7 @@ k_mark_chroma(LGCR_STAGE_ARGS) {
             row0[cx0] = 1; row0[cx1] = 1;
             row1[cx0] = 1; row1[cx1] = 1;
         }
-        if (J.listed || J.xferListed)
+        if (!pairs && (J.listed || J.xferListed))
             J.actList[warpBase + offs + __popc(bits & below)] = ((uint32_t)oy << 16) | (uint32_t)ox;
     }
 }

@@ -228,9 +228,9 @@ struct Packer {
     }
 };
 
-struct AxisOffsets { size_t start, w, wd, am, wsum, wabs, pos, lpos, cbI0, cbF, lbI0, lbF, kmx, kss, amBits; int n, sup; };
+struct AxisOffsets { size_t start, w, wd, am, wsum, wabs, pos, lpos, cbI0, cbF, lbI0, lbF, kmx, kss, amBits, pgate, nearest; int n, sup; };
 
-AxisOffsets packAxis(Packer &pk, const ChromaAxis &a) {
+AxisOffsets packAxis(Packer &pk, const ChromaAxis &a, int chromaN) {
     AxisOffsets o;
     o.n = a.n; o.sup = a.sup;
     const std::vector<double> wd(a.w.begin(), a.w.end());
@@ -249,6 +249,11 @@ AxisOffsets packAxis(Packer &pk, const ChromaAxis &a) {
             if (a.am[i * a.sup + j])
                 bits[i] |= 1u << j;
     o.amBits = pk.add(bits);
+    std::vector<float> gate;
+    std::vector<int> nearest;
+    phaseTables(a, chromaN, gate, nearest);
+    o.pgate = pk.add(gate);
+    o.nearest = pk.add(nearest);
     return o;
 }
 
@@ -264,6 +269,8 @@ AxisView axisView(const DeviceArena &ar, const AxisOffsets &o) {
     v.lbF = (const float *)ar.at(o.lbF);
     v.kmx = (const float *)ar.at(o.kmx); v.kss = (const float *)ar.at(o.kss);
     v.amBits = o.sup <= 32 ? (const uint32_t *)ar.at(o.amBits) : nullptr;
+    v.pgate = (const float *)ar.at(o.pgate);
+    v.nearest = (const int *)ar.at(o.nearest);
     return v;
 }
 
@@ -340,10 +347,36 @@ const DeviceTables *Filter::tablesFor(double shiftX, double shiftY) {
     const ChromaAxis ax = buildChromaAxis(sw, p.outW, rw, shiftX, p.k);
     const ChromaAxis ay = buildChromaAxis(sh, p.outH, rh, shiftY, p.k);
     Packer pk;
-    const AxisOffsets oax = packAxis(pk, ax), oay = packAxis(pk, ay);
+    const AxisOffsets oax = packAxis(pk, ax, cw), oay = packAxis(pk, ay, ch);
     RadialOffsets orad{};
-    if (p.k.radial)
-        orad = packRadial(pk, buildRadialTable(p.k, ax, ay, cw, ch));
+    // column pairs of the guided pass, with the jinc weights of each phase pair
+    const bool listed = p.strength > 0.0 && (p.algo == 2 || p.algo == 4);
+    const PairAxis pairs = listed ? buildPairAxis(ax, cw, float(rw)) : PairAxis{};
+    size_t opStart = 0, opBits = 0, opKind = 0, opTab = 0, opPhase = 0, opRad = 0, opRadD = 0, opSums = 0;
+    int pairPhases = 0;
+    if (pairs.sup > 0) {
+        opStart = pk.add(pairs.start);
+        opBits = pk.add(pairs.bits);
+        opKind = pk.add(pairs.kind);
+        opTab = pk.add(pairs.tab);
+    }
+    if (p.k.radial) {
+        const RadialTable rt = buildRadialTable(p.k, ax, ay, cw, ch);
+        orad = packRadial(pk, rt);
+        const PairRadial pr = buildPairRadial(rt, pairs, p.outW);
+        if (pr.valid) {
+            pairPhases = pr.phasePairs;
+            opPhase = pk.add(pr.phase);
+            opRad = pk.add(pr.w);
+            opRadD = pk.add(std::vector<double>(pr.w.begin(), pr.w.end()));
+            std::vector<double> sums;
+            for (size_t i = 0; i < rt.weightSum.size(); ++i) {
+                sums.push_back(rt.weightSum[i]);
+                sums.push_back(rt.absoluteWeightSum[i]);
+            }
+            opSums = pk.add(sums);
+        }
+    }
     const bool sameSize = p.outW == sw && p.outH == sh;
     WeightOffsets olh{}, olv{};
     if (!sameSize && !p.k.radial) {
@@ -377,8 +410,8 @@ const DeviceTables *Filter::tablesFor(double shiftX, double shiftY) {
         }
         const ChromaAxis sax = buildChromaAxis(sw, sw, rw, shiftX, p.k);
         const ChromaAxis say = buildChromaAxis(sh, sh, rh, shiftY, p.k);
-        osax = packAxis(pk, sax);
-        osay = packAxis(pk, say);
+        osax = packAxis(pk, sax, cw);
+        osay = packAxis(pk, say, ch);
         t->sAxSup = sax.sup;
         t->sAySup = say.sup;
         auto detailRowsRead = [&](int rows) {
@@ -444,6 +477,20 @@ const DeviceTables *Filter::tablesFor(double shiftX, double shiftY) {
     setAxisGeometry(*t, ax, ay, p.outH, ch);
     if (p.k.radial)
         t->rad = radialView(t->arena, orad);
+    if (pairs.sup > 0 && (!p.k.radial || pairPhases > 0)) {
+        t->pairSup = pairs.sup;
+        t->pairStart = (const int *)t->arena.at(opStart);
+        t->pairBits = (const uint32_t *)t->arena.at(opBits);
+        t->pairKind = (const int *)t->arena.at(opKind);
+        t->pairTab = (const float *)t->arena.at(opTab);
+        if (pairPhases > 0) {
+            t->pairPhases = pairPhases;
+            t->pairPhase = (const uint16_t *)t->arena.at(opPhase);
+            t->pairRad = (const float *)t->arena.at(opRad);
+            t->pairRadD = (const double *)t->arena.at(opRadD);
+            t->radSums = (const double *)t->arena.at(opSums);
+        }
+    }
     if (!sameSize && !p.k.radial) {
         t->lumaH = weightView(t->arena, olh);
         t->lumaV = weightView(t->arena, olv);
@@ -510,8 +557,18 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
     Slot sLumaTmp = take(size_t(p.outW) * sh * 4, !sameSize && !p.k.radial);  // luma / detail resize
     Slot sCnt = take(kCntCount * sizeof(unsigned long long));
     const bool listed = guided && (p.algo == 2 || p.algo == 4);
-    Slot sUvd = take(C * 16), sHTab = take(size_t(p.outW) * ch * 32, !p.k.radial);
-    Slot sWExt = take(O * 24, listed && !p.k.radial && p.k.kernel != Kernel::Bilinear);
+    // context planes of the column-pair guided pass (32 bytes per pixel) share
+    // the horizontal table's region: frames whose windows k_plain folds have no
+    // table, except the integer selector's
+    const bool pairable = listed && p.k.kernel != Kernel::Bilinear;
+    const size_t contextBytes = size_t((p.outW + 1) / 2) * 2 * p.outH * 32;    // whole pairs
+    const size_t tableBytes = p.k.radial ? 0 : size_t(p.outW) * ch * 32;
+    const bool tableKept = p.algo == 4 && !isFloat() && !p.k.radial;
+    Slot sUvd = take(C * 16);
+    Slot sHTab = take(std::max(tableBytes, pairable && !tableKept ? contextBytes : 0),
+                      !p.k.radial || pairable);
+    Slot sCtx = take(contextBytes, pairable && tableKept);
+    Slot sWExt = take(O * 24, pairable);
     Slot sList = take(O * 4, listed || (guided && p.algo == 6 && p.sparse));
     Slot sCList = take(C * 4, guided && p.algo == 6 && p.sparse);
     const bool algo6 = guided && p.algo == 6, algo4 = guided && p.algo == 4;
@@ -550,7 +607,8 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
     ws->oU = F(sOU); ws->oV = F(sOV); ws->lumaTmp = F(sLumaTmp);
     ws->counters = (unsigned long long *)ar.at(sCnt.off);
     ws->uvd = sUvd.on ? (double *)ar.at(sUvd.off) : nullptr;
-    ws->hTab = F(sHTab);
+    ws->hTab = p.k.radial ? nullptr : F(sHTab);
+    ws->context = tableKept ? F(sCtx) : pairable ? F(sHTab) : nullptr;
     ws->wExt = F(sWExt);
     ws->actList = sList.on ? (uint32_t *)ar.at(sList.off) : nullptr;
     ws->chromaList = sCList.on ? (uint32_t *)ar.at(sCList.off) : nullptr;
@@ -733,7 +791,11 @@ void buildJob(const FrameTask &t, FrameJob &J) {
     J.plainRows = J.plainFused ? T.plainRows : kPlainRowsShort;
     J.wHull = nullptr;
     J.wLum = nullptr;
-    if (ws.wExt && J.listed && J.plainFused && J.kernel != 0 && T.aySup <= 8) {
+    if (ws.wExt && J.radial) {
+        // filled by the pair form's first pass
+        J.wHull = reinterpret_cast<float4 *>(ws.wExt);
+        J.wLum = reinterpret_cast<float2 *>(ws.wExt + size_t(J.W) * J.H * 4);
+    } else if (ws.wExt && J.listed && J.plainFused && J.kernel != 0 && T.aySup <= 8) {
         // k_plain folds the guided windows' extrema for the listed pixels from
         // its staged rows; the horizontal table is then only needed for the
         // integer algo 4 plain base the guided pass recomputes
@@ -749,6 +811,31 @@ void buildJob(const FrameTask &t, FrameJob &J) {
         const int ny = (F.sh + int(J.rh) - 1) / int(J.rh);
         J.noClampX = (nx == F.cw && F.cw >= T.axSup) ? 1 : 0;
         J.noClampY = (ny == F.ch && F.ch >= T.aySup) ? 1 : 0;
+    }
+    // The guided pass can take column pairs wherever their tables exist and the
+    // taps need no clamping, bump range check or chroma-edge fade: separable
+    // frames with folded window extrema, jinc frames with the fused plain base.
+    // shapeJobs decides whether a launch does.
+    J.pairSup = 0;
+    J.guideOnGrid = J.sameSize && J.inKind != kF32;
+    if (T.pairSup > 0 && ws.context && J.listed && J.noClampX && J.noClampY && J.bumpRcpSafe && !J.cedge &&
+        T.axSup == T.aySup && (T.axSup == 4 || T.axSup == 6 || T.axSup == 8) &&
+        (J.radial ? radialPlainFused(J) : J.wHull != nullptr)) {
+        J.pairSup = T.pairSup;
+        J.context = reinterpret_cast<float4 *>(ws.context);
+        J.pairStart = T.pairStart;
+        J.pairBits = T.pairBits;
+        J.pairKind = T.pairKind;
+        J.pairTab = reinterpret_cast<const float4 *>(T.pairTab);
+        J.pairPhase = T.pairPhase;
+        J.pairPhases = T.pairPhases;
+        J.pairRad = reinterpret_cast<const float2 *>(T.pairRad);
+        J.pairRadD = reinterpret_cast<const double2 *>(T.pairRadD);
+        J.radSums = reinterpret_cast<const double2 *>(T.radSums);
+    }
+    if (J.radial && J.pairSup == 0) {
+        J.wHull = nullptr;
+        J.wLum = nullptr;
     }
     // algo 6
     J.aff = ws.aff; J.yc1 = ws.yc1; J.yc2 = ws.yc2;
@@ -977,6 +1064,9 @@ static int stageTilesShaped(const FrameJob &J, int s) {
     return 0;
 }
 
+// Fewest output pixels of a launch whose guided pass takes column pairs.
+constexpr long long kPairPixels = 1500000, kPairPixelsJinc = 400000;
+
 // Work split of the map and plain stages of one launch. Each of their blocks is
 // a serial walk (rows of a strip, words of a list, rows of a tile), so a launch
 // that leaves most SMs with less than a few blocks takes the length of one
@@ -1008,6 +1098,27 @@ void shapeJobs(FrameJob *jobs, int n) {
     const int count = longest({kCountChunk, 8192, 4096}, [](const FrameJob &J, int bytes) {
         return (long long)cdiv(J.cw * J.ch, bytes);
     });
+    // Column pairs pay where the guided pass is long enough to hide one or two
+    // more launches: measured per call, pixel form / pair form,
+    //   separable, one frame: 960x540 141 / 150 us, 1920x1080 (4:2:0, bm, bp)
+    //   678 / 655, 64 x 640x360 batched 2711 / 2636, 16 x 1080p + 16 x 4K
+    //   18690 / 18473
+    //   jinc, one frame: 640x360 123 / 130, 960x540 196 / 183, 1080p -> 4K
+    //   2379 / 2079
+    long long pixels[2] = {0, 0};
+    for (int f = 0; f < n; ++f)
+        if (jobs[f].pairSup > 0)
+            pixels[jobs[f].radial ? 1 : 0] += (long long)jobs[f].W * jobs[f].H;
+    for (int f = 0; f < n; ++f) {
+        FrameJob &J = jobs[f];
+        if (J.pairSup == 0 || pixels[J.radial ? 1 : 0] >= (J.radial ? kPairPixelsJinc : kPairPixels))
+            continue;
+        J.pairSup = 0;
+        if (J.radial) {
+            J.wHull = nullptr;
+            J.wLum = nullptr;
+        }
+    }
     const int plain = longest({kPlainRows, 32, 16, 8}, [](const FrameJob &J, int rows) {
         return (long long)cdiv(J.W, 32) * cdiv(J.H, rows);
     });
@@ -1070,7 +1181,7 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
     bool rfuse = false, ronly = !jobs.empty();
     for (const FrameJob &J : jobs) {
         rfuse = rfuse || radialPlainFused(J);
-        ronly = ronly && radialPlainFused(J);
+        ronly = ronly && (J.pairSup > 0 || radialPlainFused(J));
     }
     if (plan.totals[S_PLAIN] > 0) {
         // the dynamic shared-memory opt-in is per device (idempotent, so a
@@ -1090,7 +1201,32 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
         go(S_PLAIN, k_plain_all, b32x8, kPlainDynSmem);
     else
         go(S_PLAIN, k_plain, b32x8, kPlainDynSmem);
-    if (plan.totals[S_GUIDED] > 0) {
+    bool single = false, pairs = false, pairsRadial = false;
+    for (const FrameJob &J : jobs)
+        if (J.listed)
+            (J.pairSup == 0 ? single : J.radial ? pairsRadial : pairs) = true;
+    if (plan.totals[S_GUIDED] > 0 && (pairs || pairsRadial)) {
+        // persistent grids over the pair lists
+        using PairKernel = void (*)(const FrameJob *, const int *, int);
+        static const PairKernel kernels[4] = {k_pair_extrema, k_guide_setup, k_guided_pair,
+                                              k_guided_pair_r};
+        static int gridBlocks[4] = {0, 0, 0, 0};
+        const bool run[4] = {pairsRadial, true, pairs, pairsRadial};
+        for (int k = 0; k < 4; ++k) {
+            if (!run[k])
+                continue;
+            if (gridBlocks[k] == 0) {
+                int dev = 0, sms = 0, perSm = 0;
+                cudaGetDevice(&dev);
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernels[k], 128, 0);
+                gridBlocks[k] = std::max(1, sms * std::max(1, perSm));
+            }
+            launchAfter(kernels[k], dim3(gridBlocks[k]), dim3(128), 0, stream, dJobs, pre(S_GUIDED), n);
+            ++launches;
+        }
+    }
+    if (plan.totals[S_GUIDED] > 0 && single) {
         // persistent grid: enough resident blocks to fill every SM
         const int variant = plan.cfg.guidedVariant;
         // the instance with the fused jinc plain base when a frame needs it

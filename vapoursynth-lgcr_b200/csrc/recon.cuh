@@ -35,6 +35,8 @@ struct AxisView {
     const float *cbF, *lbF;
     const float *kmx, *kss;  // rescue kappa factors per index (separable kernels)
     const uint32_t *amBits;  // per index: bit i set when tap i is active (sup <= 32), or null
+    const float *pgate;      // per index: 1 - 2 * distance of pos to the nearest sample, or null
+    const int *nearest;      // per index: the sample nearest to pos, or null
 };
 
 struct RadialView {
@@ -68,6 +70,7 @@ enum Counter : int {
     kCntSeed = 2,
     kCntMaskPixels = 3,
     kCntRoi = 4,
+    kCntPairs = 5,           // entries of a pair list (actList of frames with pairSup > 0)
     kCntCount = 8
 };
 
@@ -127,6 +130,21 @@ struct __align__(16) FrameJob {
     double *uvd;                       // cw x ch x 2: (u, v) in FP64
     uint32_t *actList;                 // active output pixels (y << 16 | x)
     int listed;                        // frame uses the guided work list
+    // guided pass by column pairs (kernels_guided.cu): pairSup > 0 and the work
+    // list holds pairs (y << 16 | even x | 1 when only one column is active)
+    int pairSup;                       // samples of a pair's common window
+    float4 *context;                   // two per listed pixel: k_guide_setup's result
+    int guideOnGrid;                   // guide positions are luma samples (same size, integer)
+    const int *pairStart;              // per pair: first sample of the window
+    const uint32_t *pairBits;          // per pair: active taps (low half even, high half odd column)
+    const int *pairKind;               // per pair: row of pairTab
+    const float4 *pairTab;             // [kind][pairSup]: weights of both columns (separable) and
+                                       // tap distances (tap - position) * rw of both columns
+    const uint16_t *pairPhase;         // per pair: phase pair of the jinc weights
+    int pairPhases;                    // phase pairs per row phase
+    const float2 *pairRad;             // [row phase][phase pair][row][column] weights of both columns
+    const double2 *pairRadD;           // the same in FP64
+    const double2 *radSums;            // per jinc phase: sum w, sum |w|
     int listGroup;                     // work-list order: output rows per group (1: raster)
     int xferListed;                    // algo 6: detail transfer walks the work list
     uint32_t *chromaList;              // algo 6 sparse: active chroma samples (y << 16 | x)
@@ -165,7 +183,8 @@ struct __align__(16) FrameJob {
     int lgfRoiOnly;
     int blendStores;                   // the selector blend stores the typed output
     int bpStores;                      // back-projection stores the typed output
-    float *lgf;                        // 6 chroma planes: aU bU confU aV bV confV
+    float *lgf;                        // cw x ch: float4 (aU bU aV bV) per sample, then float2
+                                       // (confU confV) per sample
     float *selW2, *selW3;              // W x H routing weights (float algo 4)
     float *gU, *gV;                    // W x H guided values (float algo 4)
     uint8_t *roi;                      // cw x ch
@@ -272,6 +291,16 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+// Luma sample an output index maps to in the trust mask: floor(x * srcN / dstN).
+// Both sizes are at most 65535, so the product fits 32 bits unsigned; the
+// 64-bit division is four times as long, and resized frames take it per pixel
+// in the work list, the routing mask and the blend (one 1080p -> 4K float jinc
+// frame: k_mark_chroma 48 -> 44 us, k_roi 70 -> 67, k_blend 287 -> 215 with the
+// interleaved LGF maps).
+__device__ __forceinline__ int maskIndex(int x, int srcN, int dstN) {
+    return (int)((unsigned)x * (unsigned)srcN / (unsigned)dstN);
+}
+
 // Dilated trust mask bit of luma sample (x, y).
 __device__ __forceinline__ uint32_t maskAt(const FrameJob &J, int x, int y) {
     return (__ldg(J.mask + (size_t)y * J.maskWords + (x >> 5)) >> (x & 31)) & 1u;
@@ -384,6 +413,49 @@ __device__ __forceinline__ float footprintMean(double sum, int nx, int ny) {
     return (float)(sum / ((double)nx * (double)ny));
 }
 
+// n / d and sqrt(x) for operands that are often exactly zero (flat areas):
+// the compiler's IEEE sequences send a zero numerator or argument through
+// their out-of-line path, for the whole warp. Zero is replaced by one first
+// and the result selected, which is exact (d is never zero or NaN here when n
+// is zero).
+__device__ __forceinline__ float divZeroSafe(float n, float d) {
+    const float q = (n == 0.0f ? 1.0f : n) / d;
+    return n == 0.0f ? 0.0f : q;
+}
+__device__ __forceinline__ float sqrtZeroSafe(float x) {
+    const float r = sqrtf(x == 0.0f ? 1.0f : x);
+    return x == 0.0f ? 0.0f : r;
+}
+
+// LGF maps at a chroma position, bilinear per component: two vector loads per
+// corner instead of six scalar ones.
+struct LgfSample {
+    float4 ab;                         // aU bU aV bV
+    float2 conf;                       // confU confV
+};
+__device__ __forceinline__ float2 bilinearFast2(const float2 *p, int w, int h, int x0, float fx, int y0,
+                                                float fy) {
+    const float2 *r0 = p + (size_t)y0 * w + x0;
+    const float2 a = __ldg(r0);
+    if (w == 1) {
+        if (h == 1)
+            return a;
+        const float2 c = __ldg(r0 + 1);
+        return make_float2(a.x + (c.x - a.x) * fy, a.y + (c.y - a.y) * fy);
+    }
+    const float2 b = __ldg(r0 + 1);
+    if (h == 1)
+        return make_float2(a.x + (b.x - a.x) * fx, a.y + (b.y - a.y) * fx);
+    const float2 c = __ldg(r0 + w), d = __ldg(r0 + w + 1);
+    return make_float2(a.x + (b.x - a.x) * fx + (c.x - a.x) * fy + (a.x - b.x - c.x + d.x) * fx * fy,
+                       a.y + (b.y - a.y) * fx + (c.y - a.y) * fy + (a.y - b.y - c.y + d.y) * fx * fy);
+}
+__device__ __forceinline__ LgfSample lgfAt(const FrameJob &J, int x0, float fx, int y0, float fy) {
+    const float4 *ab = reinterpret_cast<const float4 *>(J.lgf);
+    const float2 *conf = reinterpret_cast<const float2 *>(J.lgf + 4 * (size_t)J.cw * J.ch);
+    return {bilinearFast4(ab, J.cw, J.ch, x0, fx, y0, fy), bilinearFast2(conf, J.cw, J.ch, x0, fx, y0, fy)};
+}
+
 struct TensorDir { float coherence, nx, ny; };
 
 // lgcr.h:516-538
@@ -392,8 +464,8 @@ __device__ __forceinline__ TensorDir principalDirection(float jxx, float jxy, fl
     const float difference = jxx - jyy;
     const float sum = jxx + jyy;
     const float cross = 2.0f * jxy;
-    const float disc = sqrtf(difference * difference + cross * cross);
-    d.coherence = disc / (sum + 1e-12f);
+    const float disc = sqrtZeroSafe(difference * difference + cross * cross);
+    d.coherence = divZeroSafe(disc, sum + 1e-12f);
     if (disc <= 1e-20f)
         return d;
     float vx, vy;
