@@ -44,10 +44,14 @@ struct HColumn {
     double w[SUP];
     __device__ __forceinline__ void load(const AxisView &ax, int ox) {
         tx0 = __ldg(ax.start + ox);
-        active = maskBits(ax.am + (size_t)ox * SUP, SUP);
+        active = ax.amBits ? __ldg(ax.amBits + ox) : maskBits(ax.am + (size_t)ox * SUP, SUP);
+        const double2 *src = reinterpret_cast<const double2 *>(ax.wd + (size_t)ox * SUP);
 #pragma unroll
-        for (int i = 0; i < SUP; ++i)
-            w[i] = __ldg(ax.wd + (size_t)ox * SUP + i);
+        for (int i = 0; i < SUP; i += 2) {
+            const double2 p = __ldg(src + i / 2);
+            w[i] = p.x;
+            w[i + 1] = p.y;
+        }
     }
 };
 
@@ -203,55 +207,219 @@ __device__ __forceinline__ int nthSetBit(uint32_t m, int n) {
     return pos;
 }
 
+// cp.async copies of 4, 8 and 16 bytes (both addresses aligned to the size)
+__device__ __forceinline__ void cpAsync4(void *smem, const void *gmem) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" :: "r"(dst), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cpAsync8(void *smem, const void *gmem) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(dst), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cpAsync16(void *smem, const void *gmem) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" :: "r"(dst), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cpAsyncWaitAll() {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
 // Per-row vertical tap data of one k_plain block, staged once for the
 // block's output rows (at most kPlainRows; supports up to 8 taps).
 struct PlainRows {
-    double w[kPlainRows][8];
+    double w[kPlainRows * 8];          // row by row, the axis' support apart
     int ty0[kPlainRows];
     uint32_t act[kPlainRows];
     float wsum[kPlainRows], wabs[kPlainRows], pos[kPlainRows];
     uint32_t maskWord[kPlainRows];     // active-pixel bits of the block's 32 columns
 };
 
-// The same vertical pass with the row data from PlainRows and the column
-// data (wsX, waX, posX) held in registers.
-template <int SUP, bool NOCLAMP>
-__device__ __forceinline__ void plainFromRows(const FrameJob &J, const float2 (*sHV)[32],
-                                              const float4 (*sE)[32], const PlainRows &R, int k,
-                                              int syLo, int lx, float wsX, float waX, float posX,
-                                              float &outU, float &outV) {
-    const int ty0 = R.ty0[k];
-    const uint32_t act = R.act[k];
-    double vU = 0.0, vV = 0.0;
-    float mnU = 1e30f, mxU = -1e30f, mnV = 1e30f, mxV = -1e30f;
-#pragma unroll
-    for (int j = 0; j < SUP; ++j) {
-        if (!((act >> j) & 1u))
-            continue;
-        const int r = (NOCLAMP ? ty0 + j : iclamp(ty0 + j, 0, J.ch - 1)) - syLo;
-        const float2 h = sHV[r][lx];
-        const float4 e = sE[r][lx];
-        const double w = R.w[k][j];
-        vU = fma(w, (double)h.x, vU);
-        vV = fma(w, (double)h.y, vV);
-        mnU = runMin(mnU, e.x); mxU = runMax(mxU, e.y);
-        mnV = runMin(mnV, e.z); mxV = runMax(mxV, e.w);
-    }
-    const double ws = (double)wsX * (double)R.wsum[k];
-    const double wa = (double)waX * (double)R.wabs[k];
+// The pixel's value from its vertical sums: normalised, or bilinear where the
+// weights cancel, then held to the hull. One correctly rounded reciprocal
+// serves U and V: n * r corrected by its exact remainder is the IEEE quotient
+// (Markstein, IBM J. Res. Dev. 34(1), 1990), or NaN where n or n * r is not
+// finite, and those take the division (ws, a product of two floats above 1e-6,
+// has a normal reciprocal). The hull bounds are floats and rounding is
+// monotone, so the clamp runs on the rounded value.
+__device__ __forceinline__ float2 plainValue(const FrameJob &J, double vU, double vV, float mnU, float mxU,
+                                             float mnV, float mxV, double ws, double wa, float posX,
+                                             float posY) {
+    float u, v;
     if (ws > 1e-6 && ws >= 0.05 * wa) {
-        vU /= ws;
-        vV /= ws;
+        const double r = __drcp_rn(ws);
+        const double qU = vU * r, qV = vV * r;
+        u = (float)fma(fma(-ws, qU, vU), r, qU);
+        v = (float)fma(fma(-ws, qV, vV), r, qV);
+        if (u != u || v != v) {
+            u = (float)(vU / ws);
+            v = (float)(vV / ws);
+        }
     } else {
-        vU = bilinearAt(J.U, J.cw, J.ch, posX, R.pos[k]);
-        vV = bilinearAt(J.V, J.cw, J.ch, posX, R.pos[k]);
+        u = bilinearAt(J.U, J.cw, J.ch, posX, posY);
+        v = bilinearAt(J.V, J.cw, J.ch, posX, posY);
     }
     if (J.clampHull) {
-        vU = sclamp(vU, (double)(mnU - J.margin), (double)(mxU + J.margin));
-        vV = sclamp(vV, (double)(mnV - J.margin), (double)(mxV + J.margin));
+        u = sclamp(u, mnU - J.margin, mxU + J.margin);
+        v = sclamp(v, mnV - J.margin, mxV + J.margin);
     }
-    outU = (float)vU;
-    outV = (float)vV;
+    return make_float2(u, v);
+}
+
+// Output rows k and k + 1 (two; else k alone) of one column. Their windows
+// start at most one chroma row apart, so the SUP + 1 staged rows of both are
+// read and widened once and the hull of the rows that both use is folded once.
+// Per row the order of the sums is the one-row form's.
+//  WIN 0, 1: every tap of both rows is active and no row needs clamping (the
+//  usual case away from phase 0), windows WIN rows apart: straight-line code.
+//  WIN -1: activity tested per tap.
+template <int SUP, bool NOCLAMP, int WIN>
+__device__ __forceinline__ void plainPair(const FrameJob &J, const float2 (*sHV)[32], const float4 (*sE)[32],
+                                          const PlainRows &R, int k, bool two, int syLo, int lx, float wsX,
+                                          float waX, float posX, float2 &outA, float2 &outB) {
+    const int ty0 = R.ty0[k];
+    const int kb = (WIN >= 0 || two) ? k + 1 : k;
+    const int d = WIN >= 0 ? WIN : R.ty0[kb] - ty0;
+    const uint32_t actA = WIN >= 0 ? 0u : R.act[k], actB = WIN >= 0 || !two ? 0u : R.act[kb] << d;
+    const int sup = WIN >= 0 ? SUP : J.ay.sup;
+    const double *wA = R.w + k * sup, *wB = R.w + kb * sup - d;
+    const float2 *hv = &sHV[ty0 - syLo][lx];
+    const float4 *ext = &sE[ty0 - syLo][lx];
+    double aU = 0.0, aV = 0.0, bU = 0.0, bV = 0.0;
+    float4 c = make_float4(1e30f, -1e30f, 1e30f, -1e30f), a = c, b = c;   // hulls: both rows, A only, B only
+    auto fold = [](float4 &q, const float4 &e) {
+        q.x = runMin(q.x, e.x); q.y = runMax(q.y, e.y);
+        q.z = runMin(q.z, e.z); q.w = runMax(q.w, e.w);
+    };
+#pragma unroll
+    for (int j = 0; j < SUP + (WIN == 0 ? 0 : 1); ++j) {
+        const bool inA = j < SUP && (WIN >= 0 || ((actA >> j) & 1u));
+        const bool inB = WIN >= 0 ? j >= WIN : ((actB >> j) & 1u) != 0;
+        if (!inA && !inB)
+            continue;
+        float2 h;
+        float4 e;
+        if (NOCLAMP) {
+            h = hv[j * 32];
+            e = ext[j * 32];
+        } else {
+            const int r = iclamp(ty0 + j, 0, J.ch - 1) - syLo;
+            h = sHV[r][lx];
+            e = sE[r][lx];
+        }
+        const double hU = (double)h.x, hV = (double)h.y;
+        if (inA) {
+            const double w = wA[j];
+            aU = fma(w, hU, aU);
+            aV = fma(w, hV, aV);
+        }
+        if (inB) {
+            const double w = wB[j];
+            bU = fma(w, hU, bU);
+            bV = fma(w, hV, bV);
+        }
+        if (inA && inB)
+            fold(c, e);
+        else if (inA)
+            fold(a, e);
+        else
+            fold(b, e);
+    }
+    const double dWs = (double)wsX, dWa = (double)waX;
+    fold(a, c);
+    outA = plainValue(J, aU, aV, a.x, a.y, a.z, a.w, dWs * (double)R.wsum[k], dWa * (double)R.wabs[k], posX, R.pos[k]);
+    if (WIN >= 0 || two) {
+        fold(b, c);
+        outB = plainValue(J, bU, bV, b.x, b.y, b.z, b.w, dWs * (double)R.wsum[kb], dWa * (double)R.wabs[kb], posX, R.pos[kb]);
+    }
+}
+
+template <int SUP>
+__device__ __forceinline__ void plainPairSup(const FrameJob &J, const float2 (*sHV)[32],
+                                             const float4 (*sE)[32], const PlainRows &R, int k, bool two,
+                                             int syLo, int lx, float wsX, float waX, float posX, float2 &a,
+                                             float2 &b) {
+    constexpr uint32_t kAll = (1u << SUP) - 1u;
+    if (!J.noClampY)
+        plainPair<SUP, false, -1>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b);
+    else if (two && R.act[k] == kAll && R.act[k + 1] == kAll && R.ty0[k] == R.ty0[k + 1])
+        plainPair<SUP, true, 0>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b);
+    else if (two && R.act[k] == kAll && R.act[k + 1] == kAll)
+        plainPair<SUP, true, 1>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b);
+    else
+        plainPair<SUP, true, -1>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b);
+}
+
+__device__ __forceinline__ void plainPairAny(const FrameJob &J, const float2 (*sHV)[32],
+                                             const float4 (*sE)[32], const PlainRows &R, int k, bool two,
+                                             int syLo, int lx, float wsX, float waX, float posX, float2 &a,
+                                             float2 &b) {
+    switch (J.ay.sup) {
+    case 4: plainPairSup<4>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b); break;
+    case 6: plainPairSup<6>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b); break;
+    default: plainPairSup<8>(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b); break;
+    }
+}
+
+// Chroma samples of the output rows oy (a) and, with `two`, oy + 1 (b) of one
+// column, each row to the typed output planes or to the float planes. The
+// job's fields are read once for all of them (a store would make the compiler
+// read them again).
+__device__ __forceinline__ void storePair(const FrameJob &J, bool typedA, bool typedB, int ox, int oy,
+                                          bool two, const float2 &a, const float2 &b) {
+    const bool second = two && typedB;
+    if (typedA || second) {
+        const int kind = J.outKind;
+        const long long pu = J.outPitch[1], pv = J.outPitch[2];
+        char *u = static_cast<char *>(J.out[1]) + (long long)oy * pu;
+        char *v = static_cast<char *>(J.out[2]) + (long long)oy * pv;
+        if (kind == kF32) {
+            if (typedA) {
+                reinterpret_cast<float *>(u)[ox] = a.x + 0.0f;   // s*1.0+0.0 in the reference
+                reinterpret_cast<float *>(v)[ox] = a.y + 0.0f;
+            }
+            if (second) {
+                reinterpret_cast<float *>(u + pu)[ox] = b.x + 0.0f;
+                reinterpret_cast<float *>(v + pv)[ox] = b.y + 0.0f;
+            }
+        } else {
+            const float scale = J.qScale, off = J.qOffC;
+            const int top = J.maxCode;
+            const int qa = quantize(a.x, scale, off, top), ra = quantize(a.y, scale, off, top);
+            const int qb = quantize(b.x, scale, off, top), rb = quantize(b.y, scale, off, top);
+            if (kind == kU8) {
+                if (typedA) {
+                    reinterpret_cast<uint8_t *>(u)[ox] = (uint8_t)qa;
+                    reinterpret_cast<uint8_t *>(v)[ox] = (uint8_t)ra;
+                }
+                if (second) {
+                    reinterpret_cast<uint8_t *>(u + pu)[ox] = (uint8_t)qb;
+                    reinterpret_cast<uint8_t *>(v + pv)[ox] = (uint8_t)rb;
+                }
+            } else {
+                if (typedA) {
+                    reinterpret_cast<uint16_t *>(u)[ox] = (uint16_t)qa;
+                    reinterpret_cast<uint16_t *>(v)[ox] = (uint16_t)ra;
+                }
+                if (second) {
+                    reinterpret_cast<uint16_t *>(u + pu)[ox] = (uint16_t)qb;
+                    reinterpret_cast<uint16_t *>(v + pv)[ox] = (uint16_t)rb;
+                }
+            }
+        }
+    }
+    if (!typedA || (two && !typedB)) {
+        const int W = J.W;
+        const size_t o = (size_t)oy * W + ox;
+        float *u = J.oU + o, *v = J.oV + o;
+        if (!typedA) {
+            u[0] = a.x;
+            v[0] = a.y;
+        }
+        if (two && !typedB) {
+            u[W] = b.x;
+            v[W] = b.y;
+        }
+    }
 }
 
 // Shared-memory rows of one k_plain block: float-rounded horizontal sums
@@ -352,6 +520,23 @@ __device__ __forceinline__ void extremaFromRows(const FrameJob &J, const float4 
     J.wLum[o] = make_float2(mnL, mxL);
 }
 
+__device__ __forceinline__ void foldRows(const FrameJob &J, const float4 (*sE)[32], const float2 (*sL)[32],
+                                         const PlainRows &R, int k, int syLo, int lx, size_t o) {
+    if (J.noClampY) {
+        switch (J.ay.sup) {
+        case 4: extremaFromRows<4, true>(J, sE, sL, R, k, syLo, lx, o); break;
+        case 6: extremaFromRows<6, true>(J, sE, sL, R, k, syLo, lx, o); break;
+        default: extremaFromRows<8, true>(J, sE, sL, R, k, syLo, lx, o); break;
+        }
+    } else {
+        switch (J.ay.sup) {
+        case 4: extremaFromRows<4, false>(J, sE, sL, R, k, syLo, lx, o); break;
+        case 6: extremaFromRows<6, false>(J, sE, sL, R, k, syLo, lx, o); break;
+        default: extremaFromRows<8, false>(J, sE, sL, R, k, syLo, lx, o); break;
+        }
+    }
+}
+
 // Plain stage: every pixel the guided pass does not finalize. A block covers
 // 32 output columns x J.plainRows output rows. For the separable kernels it
 // needs the horizontal entries of the chroma rows its windows touch:
@@ -362,11 +547,22 @@ __device__ __forceinline__ void extremaFromRows(const FrameJob &J, const float4 
 //    before sy, so every row some window reads is written exactly once);
 //  * other frames stage rows of the table written by k_hpass, or read the
 //    table directly when the rows do not fit (strong vertical downscale).
-// The vertical pass then runs from shared memory, with the per-row tap data
-// and active-pixel bits staged once per block for supports up to 8. Pixels
+// The vertical pass then runs from shared memory on pairs of output rows
+// (plainPair), with the per-row tap data and active-pixel bits copied there
+// while the horizontal entries are formed, for supports up to 8. Pixels
 // the guided pass lists get their window extrema folded instead (frames
 // with extrema planes), and each warp compacts its remaining plain pixels
-// across its rows so full warps evaluate them.
+// across its rows so full warps evaluate them. Blocks of 8 rows (small
+// launches) give each warp one row: pairs would leave half the warps idle.
+//
+// Bound by issue and the shared-memory pipe together (IPC 2.1, both near
+// 60 %): 64 registers and 48 KB hold it at four blocks per SM (three, with 80
+// registers: 15 % slower). One 3840x2160 10-bit frame with
+// 8-tap windows (detail transfer): 201 us by single rows with the row data
+// loaded up front, 202 with pairs alone under the activity tests, 184 with
+// straight-line pairs and the job's fields read once per store, 159 with the
+// row data copied asynchronously, 154 with the reciprocal's range test gone.
+// One 1920x1080 frame with listed pixels: 78 us before, 65 now.
 template <bool EARLY>
 __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
                                            const int *__restrict__ tileStart, int njobs) {
@@ -378,7 +574,7 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
         plainRowsSmem + size_t(kPlainStagedRows) * 32 * 24);
     __shared__ PlainRows R;
     __shared__ FrameJob sJob;
-    __shared__ uint32_t sRowBits[8][kPlainRows / 8];   // per warp: plain pixels of its rows
+    __shared__ uint32_t sRowBits[8][kPlainRows / 16][2];   // per warp: plain pixels of its row pairs
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     stageJob(jobs, f, sJob);
     const FrameJob &J = sJob;
@@ -413,18 +609,24 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
     const bool staged = (table || fused) && nRows <= kPlainStagedRows;
     const int sup = J.ay.sup;
     const bool rowTables = table && staged && sup <= 8;
+    // the row data arrive while the horizontal entries are formed
     if (rowTables) {
-        for (int i = tid; i < rowsHere * sup; i += 256) {
-            const int k = i / sup, j = i - k * sup;
-            R.w[k][j] = __ldg(J.ay.wd + (size_t)(oy0 + k) * sup + j);
-        }
-        if (tid < rowsHere) {
-            const int oy = oy0 + tid;
-            R.ty0[tid] = __ldg(J.ay.start + oy);
-            R.act[tid] = maskBits(J.ay.am + (size_t)oy * sup, sup);
-            R.wsum[tid] = __ldg(J.ay.wsum + oy);
-            R.wabs[tid] = __ldg(J.ay.wabs + oy);
-            R.pos[tid] = __ldg(J.ay.pos + oy);
+        for (int i = tid; i < rowsHere * sup; i += 256)
+            cpAsync8(R.w + i, J.ay.wd + (size_t)oy0 * sup + i);
+        const int row = tid & (kPlainRows - 1);
+        if (row < rowsHere) {
+            const int oy = oy0 + row;
+            switch (tid / kPlainRows) {
+            case 0: cpAsync4(R.ty0 + row, J.ay.start + oy); break;
+            case 1: cpAsync4(R.wsum + row, J.ay.wsum + oy); break;
+            case 2: cpAsync4(R.wabs + row, J.ay.wabs + oy); break;
+            default:
+                cpAsync4(R.pos + row, J.ay.pos + oy);
+                if (J.ay.amBits)
+                    cpAsync4(R.act + row, J.ay.amBits + oy);
+                else
+                    R.act[row] = maskBits(J.ay.am + (size_t)oy * sup, sup);
+            }
         }
     }
     // active-pixel bits: listed pixels are skipped here (after folding their
@@ -434,7 +636,7 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
     const bool needAct = skipListed || J.finalInTransfer || foldExtrema;
     const bool maskWords = needAct && J.sparse && J.sameSize;
     if (maskWords && tid < rowsHere)
-        R.maskWord[tid] = __ldg(J.mask + (size_t)(oy0 + tid) * J.maskWords + (colBase >> 5));
+        cpAsync4(R.maskWord + tid, J.mask + (size_t)(oy0 + tid) * J.maskWords + (colBase >> 5));
     if (fused) {
         // rows from the next block's first row on belong to the next block
         const int syOwnEnd = (oy0 + J.plainRows < J.H)
@@ -458,6 +660,7 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
             sE[r][lx] = make_float4(a.z, a.w, b.x, b.y);
         }
     }
+    cpAsyncWaitAll();
     __syncthreads();
     const bool colValid = ox < J.W;
     float wsX = 0.0f, waX = 0.0f, posX = 0.0f;
@@ -466,49 +669,49 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
         waX = __ldg(J.ax.wabs + ox);
         posX = __ldg(J.ax.pos + ox);
     }
+    // a warp takes pairs of rows (blocks of 8 rows: one row per warp)
+    const int per = J.plainRows >= 16 ? 2 : 1;
+    // rows k and k + 1 evaluated together: their windows start at most one row apart
+    auto twoRows = [&](int k) {
+        return per == 2 && k + 1 < rowsHere && (unsigned)(R.ty0[k + 1] - R.ty0[k]) <= 1u;
+    };
+    auto listedAt = [&](int k) {
+        return maskWords ? ((R.maskWord[k] >> lx) & 1u) != 0 : pixelActive(J, ox, oy0 + k);
+    };
     if (skipListed && rowTables) {
-        // Listed pixels only fold extrema here; the warp's plain pixels over
-        // its rows (threadIdx.y + 8m) are compacted so full warps evaluate them.
-        uint32_t *rowBits = sRowBits[threadIdx.y];
-        int total = 0;
-        for (int m = 0; m < kPlainRows / 8; ++m) {
-            const int k = threadIdx.y + 8 * m;
-            bool plainPx = false;
-            if (k < rowsHere && colValid) {
-                const int oy = oy0 + k;
-                const bool act = maskWords ? ((R.maskWord[k] >> lx) & 1u) != 0 : pixelActive(J, ox, oy);
-                if (act && foldExtrema) {
-                    const size_t o = (size_t)oy * J.W + ox;
-                    if (J.noClampY) {
-                        switch (sup) {
-                        case 4: extremaFromRows<4, true>(J, sE, sL, R, k, syLo, lx, o); break;
-                        case 6: extremaFromRows<6, true>(J, sE, sL, R, k, syLo, lx, o); break;
-                        default: extremaFromRows<8, true>(J, sE, sL, R, k, syLo, lx, o); break;
-                        }
-                    } else {
-                        switch (sup) {
-                        case 4: extremaFromRows<4, false>(J, sE, sL, R, k, syLo, lx, o); break;
-                        case 6: extremaFromRows<6, false>(J, sE, sL, R, k, syLo, lx, o); break;
-                        default: extremaFromRows<8, false>(J, sE, sL, R, k, syLo, lx, o); break;
-                        }
-                    }
+        // Listed pixels only fold extrema here; the warp's pairs with a plain
+        // pixel are compacted so full warps evaluate them.
+        uint32_t (*rowBits)[2] = sRowBits[threadIdx.y];
+        int total = 0, slot = 0;
+        for (int k0 = threadIdx.y * per; k0 < rowsHere; k0 += 8 * per, ++slot) {
+            uint32_t bits[2] = {0u, 0u};
+            for (int i = 0; i < per; ++i) {
+                const int k = k0 + i;
+                bool plainPx = false;
+                if (k < rowsHere && colValid) {
+                    const bool act = listedAt(k);
+                    if (act && foldExtrema)
+                        foldRows(J, sE, sL, R, k, syLo, lx, (size_t)(oy0 + k) * J.W + ox);
+                    plainPx = !act;
                 }
-                plainPx = !act;
+                bits[i] = __ballot_sync(0xffffffffu, plainPx);
             }
-            const uint32_t b = __ballot_sync(0xffffffffu, plainPx);
-            if (lx == 0)
-                rowBits[m] = b;
-            total += __popc(b);
+            if (lx == 0) {
+                rowBits[slot][0] = bits[0];
+                rowBits[slot][1] = bits[1];
+            }
+            total += __popc(bits[0] | bits[1]);
         }
         __syncwarp();
         for (int base = 0; base < total; base += 32) {
             const int j = base + lx;
             int m = 0, col = 0, before = 0;
             if (j < total) {
-                uint32_t b = rowBits[0];
+                uint32_t b = rowBits[0][0] | rowBits[0][1];
                 while (before + __popc(b) <= j) {
                     before += __popc(b);
-                    b = rowBits[++m];
+                    ++m;
+                    b = rowBits[m][0] | rowBits[m][1];
                 }
                 col = nthSetBit(b, j - before);
             }
@@ -516,85 +719,63 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
             const float waC = __shfl_sync(0xffffffffu, waX, col);
             const float posC = __shfl_sync(0xffffffffu, posX, col);
             if (j < total) {
-                const int k = threadIdx.y + 8 * m;
-                float u, v;
-                if (J.noClampY) {
-                    switch (sup) {
-                    case 4: plainFromRows<4, true>(J, sHV, sE, R, k, syLo, col, wsC, waC, posC, u, v); break;
-                    case 6: plainFromRows<6, true>(J, sHV, sE, R, k, syLo, col, wsC, waC, posC, u, v); break;
-                    default: plainFromRows<8, true>(J, sHV, sE, R, k, syLo, col, wsC, waC, posC, u, v); break;
-                    }
-                } else {
-                    switch (sup) {
-                    case 4: plainFromRows<4, false>(J, sHV, sE, R, k, syLo, col, wsC, waC, posC, u, v); break;
-                    case 6: plainFromRows<6, false>(J, sHV, sE, R, k, syLo, col, wsC, waC, posC, u, v); break;
-                    default: plainFromRows<8, false>(J, sHV, sE, R, k, syLo, col, wsC, waC, posC, u, v); break;
-                    }
+                const int k = (threadIdx.y + 8 * m) * per;
+                const bool onA = (rowBits[m][0] >> col) & 1u, onB = (rowBits[m][1] >> col) & 1u;
+                const bool two = onA && onB && twoRows(k);
+                // a lone plain row, or rows too far apart: one at a time
+                for (int i = onA ? 0 : 1; i < (onB && !two ? 2 : 1 + !onA); ++i) {
+                    float2 a, b = make_float2(0.0f, 0.0f);
+                    plainPairAny(J, sHV, sE, R, k + i, two, syLo, col, wsC, waC, posC, a, b);
+                    const bool typed = J.directOutput;
+                    storePair(J, typed, typed, colBase + col, oy0 + k + i, two, a, b);
                 }
-                emit(J, colBase + col, oy0 + k, u, v);
             }
         }
         return;
     }
     if (!colValid)
         return;
+    // listed pixels of a float selector or of the detail transfer: the base
+    // for what follows; other pixels: final here, or float for the next stage
+    const bool inTransfer = J.finalInTransfer, direct = J.directOutput;
+    auto typedAt = [&](bool act) { return !floatSelector && (inTransfer ? !act : direct); };
+    if (rowTables) {
+        const int end = rowsHere;
+        for (int k0 = threadIdx.y * per; k0 < end; k0 += 8 * per) {
+            const bool two = twoRows(k0);
+            for (int k = k0; ; ++k) {
+                float2 a, b = make_float2(0.0f, 0.0f);
+                plainPairAny(J, sHV, sE, R, k, two, syLo, lx, wsX, waX, posX, a, b);
+                bool actA = false, actB = false;
+                if (needAct) {
+                    actA = listedAt(k);
+                    actB = two && listedAt(k + 1);
+                    if (foldExtrema) {
+                        if (actA)
+                            foldRows(J, sE, sL, R, k, syLo, lx, (size_t)(oy0 + k) * J.W + ox);
+                        if (actB)
+                            foldRows(J, sE, sL, R, k + 1, syLo, lx, (size_t)(oy0 + k + 1) * J.W + ox);
+                    }
+                }
+                storePair(J, typedAt(actA), typedAt(actB), ox, oy0 + k, two, a, b);
+                // rows too far apart: the second by itself
+                if (two || per == 1 || k != k0 || k + 1 >= end)
+                    break;
+            }
+        }
+        return;
+    }
     for (int k = threadIdx.y; k < rowsHere; k += blockDim.y) {
-        const int oy = oy0 + k;
-        // listed pixels of algo 2 and integer algo 4 are written by k_guided
-        bool act = false;
-        if (needAct) {
-            act = maskWords ? ((R.maskWord[k] >> lx) & 1u) != 0 : pixelActive(J, ox, oy);
-            if (act && foldExtrema) {
-                const size_t o = (size_t)oy * J.W + ox;
-                if (J.noClampY) {
-                    switch (sup) {
-                    case 4: extremaFromRows<4, true>(J, sE, sL, R, k, syLo, lx, o); break;
-                    case 6: extremaFromRows<6, true>(J, sE, sL, R, k, syLo, lx, o); break;
-                    default: extremaFromRows<8, true>(J, sE, sL, R, k, syLo, lx, o); break;
-                    }
-                } else {
-                    switch (sup) {
-                    case 4: extremaFromRows<4, false>(J, sE, sL, R, k, syLo, lx, o); break;
-                    case 6: extremaFromRows<6, false>(J, sE, sL, R, k, syLo, lx, o); break;
-                    default: extremaFromRows<8, false>(J, sE, sL, R, k, syLo, lx, o); break;
-                    }
-                }
-            }
-            if (act && skipListed)
-                continue;
-        }
+        const bool act = needAct && listedAt(k);
+        if (act && skipListed)
+            continue;
         float u, v;
-        if (rowTables) {
-            if (J.noClampY) {
-                switch (sup) {
-                case 4: plainFromRows<4, true>(J, sHV, sE, R, k, syLo, lx, wsX, waX, posX, u, v); break;
-                case 6: plainFromRows<6, true>(J, sHV, sE, R, k, syLo, lx, wsX, waX, posX, u, v); break;
-                default: plainFromRows<8, true>(J, sHV, sE, R, k, syLo, lx, wsX, waX, posX, u, v); break;
-                }
-            } else {
-                switch (sup) {
-                case 4: plainFromRows<4, false>(J, sHV, sE, R, k, syLo, lx, wsX, waX, posX, u, v); break;
-                case 6: plainFromRows<6, false>(J, sHV, sE, R, k, syLo, lx, wsX, waX, posX, u, v); break;
-                default: plainFromRows<8, false>(J, sHV, sE, R, k, syLo, lx, wsX, waX, posX, u, v); break;
-                }
-            }
-        } else if (table && staged) {
-            plainFromStaged<0>(J, sHV, sE, syLo, lx, ox, oy, u, v);
-        } else {
-            plainPixel(J, ox, oy, u, v);
-        }
-        if (floatSelector || (J.finalInTransfer && act)) {
-            const size_t o = (size_t)oy * J.W + ox;
-            J.oU[o] = u;                    // base for the selector blend / detail transfer
-            J.oV[o] = v;
-            continue;
-        }
-        if (J.finalInTransfer) {
-            storeChroma(J, 1, ox, oy, u);
-            storeChroma(J, 2, ox, oy, v);
-            continue;
-        }
-        emit(J, ox, oy, u, v);
+        if (table && staged)
+            plainFromStaged<0>(J, sHV, sE, syLo, lx, ox, oy0 + k, u, v);
+        else
+            plainPixel(J, ox, oy0 + k, u, v);
+        const bool typed = typedAt(act);
+        storePair(J, typed, typed, ox, oy0 + k, false, make_float2(u, v), make_float2(u, v));
     }
 }
 
@@ -1176,18 +1357,6 @@ __device__ __forceinline__ void guidedWork(const FrameJob &J, int ox, int oy,
 // are the same either way.
 constexpr int kGuidedMaxFrames = 1024;
 
-// cp.async copies of 4 and 16 bytes (both addresses aligned to the size)
-__device__ __forceinline__ void cpAsync4(void *smem, const void *gmem) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" :: "r"(dst), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cpAsync16(void *smem, const void *gmem) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" :: "r"(dst), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cpAsyncWaitAll() {
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
 
 static_assert(kGuidedStageBytes == size_t(8) * kStageRows * kStageCols * (4 + 16),
               "staged guided windows: 8 warps x kStageRows x kStageCols x (lc + (u, v))");
