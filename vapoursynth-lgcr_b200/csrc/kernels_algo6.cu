@@ -407,36 +407,83 @@ __device__ __forceinline__ void detailEntry(const float *row, int cw, int tx0, c
     ext = make_float2(lo, hi);
 }
 
-template <bool NOCLAMP>
-__device__ __forceinline__ double detailVertical(const DetailRows &R, const double (*sH)[32],
-                                                 const float2 (*sE)[32], int k, int lx, int syLo,
-                                                 int ch, float &mn, float &mx) {
+// Vertical sums and extrema of the tile rows k (a) and k + 1 (b, with `two`)
+// of one column, as the plain stage forms its row pairs: the SUP + 1 staged
+// rows of both windows are read once. WIN 0, 1: every tap of both rows active,
+// none clamped, windows WIN rows apart; WIN -1: activity tested per tap.
+struct DetailSum { double v; float lo, hi; };
+
+template <int SUP, bool NOCLAMP, int WIN>
+__device__ __forceinline__ void detailPair(const DetailRows &R, const double (*sH)[32],
+                                           const float2 (*sE)[32], int k, bool two, int lx, int syLo,
+                                           int ch, DetailSum &a, DetailSum &b) {
     const int ty0 = R.ty0[k];
-    const uint32_t act = R.act[k];
-    double v = 0.0;
-    float lo = 1e30f, hi = -1e30f;
+    const int kb = (WIN >= 0 || two) ? k + 1 : k;
+    const int d = WIN >= 0 ? WIN : R.ty0[kb] - ty0;
+    const uint32_t actA = WIN >= 0 ? 0u : R.act[k], actB = WIN >= 0 || !two ? 0u : R.act[kb] << d;
+    const double *wA = R.w[k], *wB = R.w[kb] - d;
+    const double *hv = &sH[ty0 - syLo][lx];
+    const float2 *ext = &sE[ty0 - syLo][lx];
+    float lo = 1e30f, hi = -1e30f;                          // rows that both use
+    a.v = b.v = 0.0;
+    a.lo = b.lo = 1e30f;
+    a.hi = b.hi = -1e30f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (!((act >> j) & 1u))
+    for (int j = 0; j < SUP + (WIN == 0 ? 0 : 1); ++j) {
+        const bool inA = j < SUP && (WIN >= 0 || ((actA >> j) & 1u));
+        const bool inB = WIN >= 0 ? j >= WIN : ((actB >> j) & 1u) != 0;
+        if (!inA && !inB)
             continue;
-        const int r = (NOCLAMP ? ty0 + j : iclamp(ty0 + j, 0, ch - 1)) - syLo;
-        v = fma(R.w[k][j], sH[r][lx], v);
-        const float2 e = sE[r][lx];
-        lo = runMin(lo, e.x);
-        hi = runMax(hi, e.y);
+        const int r = NOCLAMP ? 0 : iclamp(ty0 + j, 0, ch - 1) - syLo;
+        const double h = NOCLAMP ? hv[j * 32] : sH[r][lx];
+        const float2 e = NOCLAMP ? ext[j * 32] : sE[r][lx];
+        if (inA)
+            a.v = fma(wA[j], h, a.v);
+        if (inB)
+            b.v = fma(wB[j], h, b.v);
+        if (inA && inB) {
+            lo = runMin(lo, e.x);
+            hi = runMax(hi, e.y);
+        } else if (inA) {
+            a.lo = runMin(a.lo, e.x);
+            a.hi = runMax(a.hi, e.y);
+        } else {
+            b.lo = runMin(b.lo, e.x);
+            b.hi = runMax(b.hi, e.y);
+        }
     }
-    mn = lo;
-    mx = hi;
-    return v;
+    a.lo = runMin(a.lo, lo);
+    a.hi = runMax(a.hi, hi);
+    b.lo = runMin(b.lo, lo);
+    b.hi = runMax(b.hi, hi);
 }
 
-__global__ void __launch_bounds__(256)
+template <int SUP>
+__device__ __forceinline__ void detailPairSup(const DetailRows &R, const double (*sH)[32],
+                                              const float2 (*sE)[32], int k, bool two, int lx, int syLo,
+                                              int ch, bool noClamp, DetailSum &a, DetailSum &b) {
+    constexpr uint32_t kAll = (1u << SUP) - 1u;
+    const bool full = two && R.act[k] == kAll && R.act[k + 1] == kAll;
+    if (!noClamp)
+        detailPair<SUP, false, -1>(R, sH, sE, k, two, lx, syLo, ch, a, b);
+    else if (full && R.ty0[k] == R.ty0[k + 1])
+        detailPair<SUP, true, 0>(R, sH, sE, k, two, lx, syLo, ch, a, b);
+    else if (full)
+        detailPair<SUP, true, 1>(R, sH, sE, k, two, lx, syLo, ch, a, b);
+    else
+        detailPair<SUP, true, -1>(R, sH, sE, k, two, lx, syLo, ch, a, b);
+}
+
+// Bound by latency and issue (IPC 2 at four blocks per SM). One 3840x2160
+// frame with 8-tap windows: 175 us by single rows at three blocks per SM with
+// the row data loaded up front and the horizontal Nyquist pass through shared
+// memory, 125 us now (five blocks at 48 registers, which spill: 132).
+__global__ void __launch_bounds__(256, 4)
 k_detail_map(LGCR_STAGE_ARGS) {
     gridDependency();
     __shared__ double sH[kDetailStagedRows][32];
     __shared__ float2 sE[kDetailStagedRows][32];
     __shared__ float sD[kDetailRowsTall + 2][33];
-    __shared__ float sX[kDetailRowsTall + 2][33];
     __shared__ DetailRows R;
     __shared__ FrameJob sJob;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
@@ -470,19 +517,29 @@ k_detail_map(LGCR_STAGE_ARGS) {
     const int c = iclamp(x0 - 1 + lx, 0, w - 1);
     const AxisView &ax = J.sax, &ay = J.say;
     const int supY = ay.sup;
-    for (int i = tid; i < rowsIn * supY; i += 256) {
-        const int k = i / supY, j = i - k * supY;
-        const int rk = iclamp(y0 - 1 + k, 0, h - 1);
-        R.w[k][j] = __ldg(ay.wd + (size_t)rk * supY + j);
+    // the row data arrive while the horizontal entries are formed
+    for (int i = tid; i < rowsIn * 8; i += 256) {
+        const int k = i >> 3, j = i & 7;
+        if (j < supY)
+            cpAsync8(&R.w[k][j], ay.wd + (size_t)iclamp(y0 - 1 + k, 0, h - 1) * supY + j);
     }
-    if (tid < rowsIn) {
-        const int rk = iclamp(y0 - 1 + tid, 0, h - 1);
-        R.r[tid] = rk;
-        R.ty0[tid] = __ldg(ay.start + rk);
-        R.act[tid] = activityBits(ay.am + (size_t)rk * supY, supY);
-        R.wsum[tid] = __ldg(ay.wsum + rk);
-        R.wabs[tid] = __ldg(ay.wabs + rk);
-        R.pos[tid] = __ldg(ay.pos + rk);
+    static_assert(kDetailRowsTall + 2 == 64, "four groups of 64 threads fetch the row data");
+    if ((tid & 63) < rowsIn) {
+        const int k = tid & 63, rk = iclamp(y0 - 1 + k, 0, h - 1);
+        switch (tid >> 6) {
+        case 0:
+            cpAsync4(R.ty0 + k, ay.start + rk);
+            R.r[k] = rk;
+            break;
+        case 1: cpAsync4(R.wsum + k, ay.wsum + rk); break;
+        case 2: cpAsync4(R.wabs + k, ay.wabs + rk); break;
+        default:
+            cpAsync4(R.pos + k, ay.pos + rk);
+            if (ay.amBits)
+                cpAsync4(R.act + k, ay.amBits + rk);
+            else
+                R.act[k] = activityBits(ay.am + (size_t)rk * supY, supY);
+        }
     }
     const int syLo = iclamp(__ldg(ay.start + iclamp(y0 - 1, 0, h - 1)), 0, ch - 1);
     const int syHi = iclamp(__ldg(ay.start + iclamp(y0 + rowsOut, 0, h - 1)) + supY - 1, 0, ch - 1);
@@ -492,7 +549,7 @@ k_detail_map(LGCR_STAGE_ARGS) {
         // horizontal entries of column c on the chroma rows the tile reads
         const int supX = ax.sup;
         const int tx0 = __ldg(ax.start + c);
-        const uint32_t act = activityBits(ax.am + (size_t)c * supX, supX);
+        const uint32_t act = ax.amBits ? __ldg(ax.amBits + c) : activityBits(ax.am + (size_t)c * supX, supX);
         double wx[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -509,44 +566,61 @@ k_detail_map(LGCR_STAGE_ARGS) {
             sE[r][lx] = e;
         }
     }
+    cpAsyncWaitAll();
     __syncthreads();
     {
         const float wsX = __ldg(ax.wsum + c), waX = __ldg(ax.wabs + c), posX = __ldg(ax.pos + c);
-        for (int k = threadIdx.y; k < rowsIn; k += blockDim.y) {
-            float mn, mx;
-            double v = J.sNoClampY ? detailVertical<true>(R, sH, sE, k, lx, syLo, ch, mn, mx)
-                                   : detailVertical<false>(R, sH, sE, k, lx, syLo, ch, mn, mx);
+        const bool noClamp = J.sNoClampY, clampHull = J.clampHull, nyqX = J.nyqX;
+        const float margin = J.margin;
+        const float *Y = J.Y + c;
+        // one row's detail sample to the tile, after the horizontal Nyquist
+        // pass on the warp's row where there is one
+        auto finish = [&](int k, const DetailSum &q) {
             const double ws = (double)wsX * (double)R.wsum[k];
             const double wa = (double)waX * (double)R.wabs[k];
+            float v;
             if (ws > 1e-6 && ws >= 0.05 * wa)
-                v /= ws;
+                v = (float)(q.v / ws);
             else
                 v = bilinearAt(dgl, cw, ch, posX, R.pos[k]);
-            if (J.clampHull)
-                v = sclamp(v, (double)(mn - J.margin), (double)(mx + J.margin));
-            sD[k][lx] = ldf(J.Y + (size_t)R.r[k] * w + c) - (float)v;
+            if (clampHull)
+                v = sclamp(v, q.lo - margin, q.hi + margin);
+            float dv = ldf(Y + (size_t)R.r[k] * w) - v;
+            if (nyqX) {
+                const float left = __shfl_up_sync(0xffffffffu, dv, 1), right = __shfl_down_sync(0xffffffffu, dv, 1);
+                dv = 0.25f * left + 0.5f * dv + 0.25f * right;
+            }
+            sD[k][lx] = dv;
+        };
+        for (int k0 = threadIdx.y * 2; k0 < rowsIn; k0 += 16) {
+            // rowsIn is even; windows further apart go one at a time
+            const bool two = (unsigned)(R.ty0[k0 + 1] - R.ty0[k0]) <= 1u;
+            for (int k = k0; ; ++k) {
+                DetailSum a, b;
+                switch (supY) {
+                case 4: detailPairSup<4>(R, sH, sE, k, two, lx, syLo, ch, noClamp, a, b); break;
+                case 6: detailPairSup<6>(R, sH, sE, k, two, lx, syLo, ch, noClamp, a, b); break;
+                default: detailPairSup<8>(R, sH, sE, k, two, lx, syLo, ch, noClamp, a, b); break;
+                }
+                finish(k, a);
+                if (two)
+                    finish(k + 1, b);
+                if (two || k != k0)
+                    break;
+            }
         }
     }
     __syncthreads();
-    const float (*src)[33] = sD;
-    if (J.nyqX) {
-        if (lx >= 1 && lx <= kDetailTile)
-            for (int k = threadIdx.y; k < rowsIn; k += blockDim.y)
-                sX[k][lx] = 0.25f * sD[k][lx - 1] + 0.5f * sD[k][lx] + 0.25f * sD[k][lx + 1];
-        __syncthreads();
-        src = sX;
-    }
     const int x = x0 - 1 + lx;
     if (lx < 1 || lx > kDetailTile || x >= w)
         return;
-    float *dst = const_cast<float *>(J.detailSrc);
+    float *dst = const_cast<float *>(J.detailSrc) + x;
+    const bool nyqY = J.nyqY;
     for (int k = 1 + threadIdx.y; k <= rowsOut; k += blockDim.y) {
         const int y = y0 - 1 + k;
         if (y >= h)
             break;
-        const float val = J.nyqY ? 0.25f * src[k - 1][lx] + 0.5f * src[k][lx] + 0.25f * src[k + 1][lx]
-                                 : src[k][lx];
-        dst[(size_t)y * w + x] = val;
+        dst[(size_t)y * w] = nyqY ? 0.25f * sD[k - 1][lx] + 0.5f * sD[k][lx] + 0.25f * sD[k + 1][lx] : sD[k][lx];
     }
 }
 

@@ -207,23 +207,6 @@ __device__ __forceinline__ int nthSetBit(uint32_t m, int n) {
     return pos;
 }
 
-// cp.async copies of 4, 8 and 16 bytes (both addresses aligned to the size)
-__device__ __forceinline__ void cpAsync4(void *smem, const void *gmem) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" :: "r"(dst), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cpAsync8(void *smem, const void *gmem) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(dst), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cpAsync16(void *smem, const void *gmem) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" :: "r"(dst), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cpAsyncWaitAll() {
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
 // Per-row vertical tap data of one k_plain block, staged once for the
 // block's output rows (at most kPlainRows; supports up to 8 taps).
 struct PlainRows {

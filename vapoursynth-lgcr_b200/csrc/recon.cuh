@@ -229,6 +229,23 @@ __device__ __forceinline__ float runMax(float acc, float v) { return fmaxf(acc, 
 __device__ __forceinline__ double runMin(double acc, double v) { return (v < acc) ? v : acc; }
 __device__ __forceinline__ double runMax(double acc, double v) { return (acc < v) ? v : acc; }
 
+// cp.async copies of 4, 8 and 16 bytes (both addresses aligned to the size)
+__device__ __forceinline__ void cpAsync4(void *smem, const void *gmem) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" :: "r"(dst), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cpAsync8(void *smem, const void *gmem) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(dst), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cpAsync16(void *smem, const void *gmem) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" :: "r"(dst), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cpAsyncWaitAll() {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
 __device__ __forceinline__ float ldf(const float *p) { return __ldg(p); }
 
 // 1/x for denominators of the form 1 + (non-negative terms), i.e. x >= 1,
