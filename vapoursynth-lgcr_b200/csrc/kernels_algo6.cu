@@ -63,6 +63,13 @@ __global__ void k_yc_h(LGCR_STAGE_ARGS) {
 // sums of every luma row the tile reads go to shared memory once (per
 // candidate), then each sample runs its vertical pass from there. Same
 // operands and order as candidateAt. Tap supports up to 8.
+//
+// Bound by the integer pipe (clamped indices) and the widening conversions.
+// Chroma at half the luma's width gives 4 taps inside the 8 of the second
+// candidate: away from the plane's sides one read and one widening of the 8
+// samples then serve both. The vertical weights are widened once per tile. One
+// 3840x2160 4:2:0 frame: 98 us with every tap read, clamped and widened by
+// itself, 60 us now (five blocks per SM at 48 registers; four: 67, three: 75).
 __device__ __forceinline__ float ycHorizontal(const FrameJob &J, const WeightView &th, int cx, int row,
                                               const double (&w)[8], int s0) {
     const float *lrow = J.Y + (size_t)row * J.sw;
@@ -74,23 +81,30 @@ __device__ __forceinline__ float ycHorizontal(const FrameJob &J, const WeightVie
     return (float)hv;
 }
 
-__device__ __forceinline__ float ycVertical(const FrameJob &J, const WeightView &tv, int cy,
-                                            const float (*sH)[32], int lo, int lx) {
-    const int sv = __ldg(tv.start + cy);
-    const float *wv = tv.w + (size_t)cy * tv.sup;
+struct YcRows {
+    double w[kYcTile][8];
+    int start[kYcTile];
+};
+
+template <bool INNER>
+__device__ __forceinline__ float ycVertical(const YcRows &R, int k, int sup, int sh, const float (*sH)[32],
+                                            int lo, int lx) {
+    const int sv = R.start[k];
+    const float *col = &sH[sv - lo][lx];
     double acc = 0.0;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        if (j < tv.sup)
-            acc = fma((double)__ldg(wv + j), (double)sH[iclamp(sv + j, 0, J.sh - 1) - lo][lx], acc);
+        if (j < sup)
+            acc = fma(R.w[k][j], (double)(INNER ? col[j * 32] : sH[iclamp(sv + j, 0, sh - 1) - lo][lx]), acc);
     return (float)acc;
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 k_yc_tiled(LGCR_STAGE_ARGS) {
     gridDependency();
     __shared__ float sH1[kYcRows][32];
     __shared__ float sH2[kYcRows][32];
+    __shared__ YcRows R1, R2;
     __shared__ FrameJob sJob;
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     stageJob(jobs, f, sJob);
@@ -102,40 +116,100 @@ k_yc_tiled(LGCR_STAGE_ARGS) {
     const int lx = threadIdx.x;
     const int cx = cx0 + lx;
     const int cxc = min(cx, J.cw - 1);
-    const int lo1 = iclamp(__ldg(J.ycV1.start + cy0), 0, J.sh - 1);
-    const int hi1 = iclamp(__ldg(J.ycV1.start + cyLast) + J.ycV1.sup - 1, 0, J.sh - 1);
-    const int lo2 = iclamp(__ldg(J.ycV2.start + cy0), 0, J.sh - 1);
-    const int hi2 = iclamp(__ldg(J.ycV2.start + cyLast) + J.ycV2.sup - 1, 0, J.sh - 1);
+    const int sw = J.sw, sh = J.sh;
+    const int supH1 = J.ycH1.sup, supH2 = J.ycH2.sup, supV1 = J.ycV1.sup, supV2 = J.ycV2.sup;
+    const int lo1 = iclamp(__ldg(J.ycV1.start + cy0), 0, sh - 1);
+    const int hi1 = iclamp(__ldg(J.ycV1.start + cyLast) + supV1 - 1, 0, sh - 1);
+    const int lo2 = iclamp(__ldg(J.ycV2.start + cy0), 0, sh - 1);
+    const int hi2 = iclamp(__ldg(J.ycV2.start + cyLast) + supV2 - 1, 0, sh - 1);
+    {
+        // vertical weights of the tile's rows
+        static_assert(kYcTile * 8 == 256, "one weight per thread and candidate");
+        const int tid = threadIdx.y * 32 + lx, k = tid >> 3, j = tid & 7;
+        const int cy = min(cy0 + k, J.ch - 1);
+        if (j < supV1)
+            R1.w[k][j] = (double)__ldg(J.ycV1.w + (size_t)cy * supV1 + j);
+        if (j < supV2)
+            R2.w[k][j] = (double)__ldg(J.ycV2.w + (size_t)cy * supV2 + j);
+        if (j == 0) {
+            R1.start[k] = __ldg(J.ycV1.start + cy);
+            R2.start[k] = __ldg(J.ycV2.start + cy);
+        }
+    }
     {
         double w1[8], w2[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            w1[i] = i < J.ycH1.sup ? (double)__ldg(J.ycH1.w + (size_t)cxc * J.ycH1.sup + i) : 0.0;
-            w2[i] = i < J.ycH2.sup ? (double)__ldg(J.ycH2.w + (size_t)cxc * J.ycH2.sup + i) : 0.0;
+            w1[i] = i < supH1 ? (double)__ldg(J.ycH1.w + (size_t)cxc * supH1 + i) : 0.0;
+            w2[i] = i < supH2 ? (double)__ldg(J.ycH2.w + (size_t)cxc * supH2 + i) : 0.0;
         }
         const int s1 = __ldg(J.ycH1.start + cxc), s2 = __ldg(J.ycH2.start + cxc);
-        for (int r = threadIdx.y; r <= hi1 - lo1; r += blockDim.y)
-            sH1[r][lx] = ycHorizontal(J, J.ycH1, cxc, lo1 + r, w1, s1);
-        for (int r = threadIdx.y; r <= hi2 - lo2; r += blockDim.y)
-            sH2[r][lx] = ycHorizontal(J, J.ycH2, cxc, lo2 + r, w2, s2);
+        const bool nested = supH1 == 4 && supH2 == 8 && s1 == s2 + 2 && s2 >= 0 && s2 + 7 < sw;
+        if (lo2 <= lo1 && hi1 <= hi2 && __all_sync(0xffffffffu, nested)) {
+            const float *col = J.Y + s2;
+            for (int r = lo2 + threadIdx.y; r <= hi2; r += blockDim.y) {
+                const float *p = col + (size_t)r * sw;
+                double h1 = 0.0, h2 = 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const double d = (double)ldf(p + i);
+                    h2 = fma(w2[i], d, h2);
+                    if (i >= 2 && i < 6)
+                        h1 = fma(w1[i - 2], d, h1);
+                }
+                sH2[r - lo2][lx] = (float)h2;
+                if (r >= lo1 && r <= hi1)
+                    sH1[r - lo1][lx] = (float)h1;
+            }
+        } else {
+            for (int r = threadIdx.y; r <= hi1 - lo1; r += blockDim.y)
+                sH1[r][lx] = ycHorizontal(J, J.ycH1, cxc, lo1 + r, w1, s1);
+            for (int r = threadIdx.y; r <= hi2 - lo2; r += blockDim.y)
+                sH2[r][lx] = ycHorizontal(J, J.ycH2, cxc, lo2 + r, w2, s2);
+        }
     }
     __syncthreads();
     if (cx >= J.cw)
         return;
     const size_t C = (size_t)J.cw * J.ch;
+    float *out1 = J.yc1, *out2 = J.yc2, *consensus = J.aff + 8 * C;
+    const float *lc = J.lc;
+    const int cw = J.cw;
     for (int k = threadIdx.y; cy0 + k <= cyLast; k += blockDim.y) {
-        const int cy = cy0 + k;
-        const size_t o = (size_t)cy * J.cw + cx;
-        const float y1 = ycVertical(J, J.ycV1, cy, sH1, lo1, lx);
-        const float y2 = ycVertical(J, J.ycV2, cy, sH2, lo2, lx);
-        J.yc1[o] = y1;
-        J.yc2[o] = y2;
-        J.aff[8 * C + o] = median3f(ldf(J.lc + o), y1, y2);   // degraded luma consensus
+        const size_t o = (size_t)(cy0 + k) * cw + cx;
+        const bool inner = R1.start[k] >= 0 && R2.start[k] >= 0 && R1.start[k] + supV1 <= sh &&
+                           R2.start[k] + supV2 <= sh;
+        const float y1 = inner ? ycVertical<true>(R1, k, supV1, sh, sH1, lo1, lx)
+                               : ycVertical<false>(R1, k, supV1, sh, sH1, lo1, lx);
+        const float y2 = inner ? ycVertical<true>(R2, k, supV2, sh, sH2, lo2, lx)
+                               : ycVertical<false>(R2, k, supV2, sh, sH2, lo2, lx);
+        out1[o] = y1;
+        out2[o] = y2;
+        consensus[o] = median3f(ldf(lc + o), y1, y2);   // degraded luma consensus
     }
 }
 
+// Quotients n / d of one denominator, from its correctly rounded reciprocal r:
+// n * r corrected by its exact remainder is the IEEE quotient (Markstein, IBM
+// J. Res. Dev. 34(1), 1990), or NaN where n or n * r is not finite, and that
+// takes the division itself (out of line: its code and registers stay out of
+// the caller).
+__device__ __noinline__ double quotientCold(double n, double d) { return n / d; }
+__device__ __forceinline__ double quotientBy(double n, double d, double r) {
+    const double q = n * r;
+    const double v = fma(fma(-d, q, n), r, q);
+    if (v == v)
+        return v;
+    return quotientCold(n, d);
+}
+
 // 5x5 affine statistics of one chroma sample (buildAffineMaps,
-// src/algos.cpp:1026-1526).
+// src/algos.cpp:1026-1526). Bound by the FP64 pipe and the widening
+// conversions: a product of two floats is exact in double, so one fused
+// multiply-add rounds as the multiply and the add did, and the means share the
+// reciprocal of their count. The list form on one 3840x2160 4:2:0 frame: 107 us
+// with separate products and a division per mean, 90 us now (four blocks per
+// SM, which spill: 113; two: 96).
 __device__ __forceinline__ bool affineSparse(const FrameJob &J) {
     return J.sparse && (unsigned long long)J.counters[kCntActiveChroma] * 2ull <
                            (unsigned long long)J.cw * J.ch;
@@ -150,19 +224,22 @@ __device__ __forceinline__ void affineSample(const FrameJob &J, int x, int y, bo
     double s[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) s[k] = 0.0;
-    float mnU = ldf(J.U + (size_t)top * w + left), mxU = mnU;
-    float mnV = ldf(J.V + (size_t)top * w + left), mxV = mnV;
+    const float firstU = ldf(J.U + (size_t)top * w + left), firstV = ldf(J.V + (size_t)top * w + left);
+    float mnU = firstU, mxU = firstU, mnV = firstV, mxV = firstV;
     auto tap = [&](size_t q) {
         const float uf = ldf(J.U + q), vf = ldf(J.V + q);
         const double u = uf, v = vf;
-        s[0] += u; s[1] += u * u; s[2] += v; s[3] += v * v;
-        mnU = smin(mnU, uf); mxU = smax(mxU, uf);
-        mnV = smin(mnV, vf); mxV = smax(mxV, vf);
+        s[0] += u; s[1] = fma(u, u, s[1]); s[2] += v; s[3] = fma(v, v, s[3]);
+        mnU = runMin(mnU, uf); mxU = runMax(mxU, uf);
+        mnV = runMin(mnV, vf); mxV = runMax(mxV, vf);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const double ly = ldf(yc[k] + q);
             const int b = 4 + 4 * k;
-            s[b] += ly; s[b + 1] += ly * ly; s[b + 2] += ly * u; s[b + 3] += ly * v;
+            s[b] += ly;
+            s[b + 1] = fma(ly, ly, s[b + 1]);
+            s[b + 2] = fma(ly, u, s[b + 2]);
+            s[b + 3] = fma(ly, v, s[b + 3]);
         }
     };
     if (bottom - top == 4 && right - left == 4) {
@@ -178,11 +255,16 @@ __device__ __forceinline__ void affineSample(const FrameJob &J, int x, int y, bo
             for (int px = left; px <= right; ++px)
                 tap((size_t)py * w + px);
     }
+    // a NaN first sample stays the extremum (the comparisons with it fail)
+    if (firstU != firstU)
+        mnU = mxU = firstU;
+    if (firstV != firstV)
+        mnV = mxV = firstV;
     const int n = (right - left + 1) * (bottom - top + 1);
     const double eps = J.lgfEps;
     const double epsSig = J.epsSig;
     const double inv = 1.0 / n;
-    auto mean = [&](double sum) { return sparseRoi ? sum * inv : sum / n; };
+    auto mean = [&](double sum) { return sparseRoi ? sum * inv : quotientBy(sum, (double)n, inv); };
     const double meanU = mean(s[0]), meanV = mean(s[2]);
     const double varU = smax(0.0, mean(s[1]) - meanU * meanU);
     const double varV = smax(0.0, mean(s[3]) - meanV * meanV);
@@ -194,8 +276,9 @@ __device__ __forceinline__ void affineSample(const FrameJob &J, int x, int y, bo
         const double varY = smax(0.0, mean(s[b + 1]) - meanY * meanY);
         const double covU = mean(s[b + 2]) - meanY * meanU;
         const double covV = mean(s[b + 3]) - meanY * meanV;
-        aU[k] = sclamp(covU / (varY + eps), -16.0, 16.0);
-        aV[k] = sclamp(covV / (varY + eps), -16.0, 16.0);
+        const double dY = varY + eps;
+        aU[k] = sclamp(covU / dY, -16.0, 16.0);
+        aV[k] = sclamp(covV / dY, -16.0, 16.0);
         q[k] = sclamp((covU * covU + covV * covV) / ((varY + eps) * (varU + varV + eps)), 0.0, 1.0);
     }
     const size_t C = (size_t)w * h;
