@@ -708,6 +708,10 @@ __device__ __forceinline__ float gateAt(const GateTile &T, int x, int y, int x0,
         return 0.0f;
     const TensorDir dir = principalDirection(sxx, sxy, syy);
     const float nx = dir.nx, ny = dir.ny;
+    // the direction of non-finite gradients is NaN and so is every sum below;
+    // its positions would index outside the tile
+    if (!(fabsf(nx) <= 1.5f && fabsf(ny) <= 1.5f))
+        return __int_as_float(0x7fffffff);
     // moments of (gY, gC) as packed pairs: sum, sum of squares, k-weighted sum
     const f32x2 nx2 = pk2(nx, nx), ny2 = pk2(ny, ny);
     f32x2 sum2 = pk2(0.0f, 0.0f), sq2 = sum2, mom2 = sum2;
