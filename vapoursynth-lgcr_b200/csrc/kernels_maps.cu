@@ -239,7 +239,7 @@ __device__ __forceinline__ void convertChroma(const FrameJob &J, int cy, int xb,
     }
 }
 
-__global__ void __launch_bounds__(kConvertWarps * 32, 3)
+__global__ void __launch_bounds__(kConvertWarps * 32, 5)
 k_convert(LGCR_STAGE_ARGS) {
     gridDependency();
     __shared__ FrameJob sJob;
