@@ -1071,84 +1071,121 @@ k_lgf(LGCR_STAGE_ARGS) {
     storeLgf(J, o, ab, make_float2(confU, confV));
 }
 
+// Walk of the selector's routing and blend stages: a block covers 32 output
+// columns x J.plainRows rows, a thread one column, so the frame lookup, the
+// job's fields and the column's mask, chroma and luma positions are found once
+// per thread and not once per sample. Both wait for loads, so they take 32
+// registers (eight blocks per SM) although the blend spills a few. One pixel
+// per thread took, for one 1920x1080 -> 3840x2160 float frame, 67 us (routing)
+// and 214 us (blend); 48 and 156 us now (the blend with 64 registers 201, 48
+// 174, 40 177).
+struct ColumnWalk {
+    int ox, oy, end;                   // column, first and past-the-last row of the thread
+    int mx;                            // the column in the mask
+    bool valid;
+    __device__ __forceinline__ ColumnWalk(const FrameJob &J, int tile) {
+        const int tilesX = (J.W + 31) >> 5, ty = tile / tilesX;
+        ox = (tile - ty * tilesX) * 32 + threadIdx.x;
+        oy = ty * J.plainRows + threadIdx.y;
+        end = min(ty * J.plainRows + J.plainRows, J.H);
+        valid = ox < J.W;
+        mx = J.sameSize || !valid ? ox : min(J.sw - 1, maskIndex(ox, J.sw, J.W));
+    }
+    __device__ __forceinline__ bool active(const FrameJob &J, int y) const {
+        return !J.sparse || maskAt(J, mx, J.sameSize ? y : min(J.sh - 1, maskIndex(y, J.sh, J.H))) != 0;
+    }
+};
+
 // Mark the 2x2 chroma footprint of output samples whose diagonal routing
 // weight reaches 1e-4.
-__global__ void k_roi(LGCR_STAGE_ARGS) {
+__global__ void __launch_bounds__(256, 8)
+k_roi(LGCR_STAGE_ARGS) {
     gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
-    int ox, oy;
-    tile32x8(blockIdx.x - tileStart[f], J.W, ox, oy);
-    if (ox >= J.W || oy >= J.H || !activeOut(J, ox, oy))
+    const ColumnWalk c(J, blockIdx.x - tileStart[f]);
+    if (!c.valid)
         return;
-    if (J.selW3[(size_t)oy * J.W + ox] < 1e-4f)
-        return;
-    const int cx0 = __ldg(J.ax.cbI0 + ox), cx1 = min(cx0 + 1, J.cw - 1);
-    const int cy0 = __ldg(J.ay.cbI0 + oy), cy1 = min(cy0 + 1, J.ch - 1);
-    J.roi[(size_t)cy0 * J.cw + cx0] = 1;
-    J.roi[(size_t)cy0 * J.cw + cx1] = 1;
-    J.roi[(size_t)cy1 * J.cw + cx0] = 1;
-    J.roi[(size_t)cy1 * J.cw + cx1] = 1;
+    const int cw = J.cw, cyMax = J.ch - 1;
+    const int cx0 = __ldg(J.ax.cbI0 + c.ox), cx1 = min(cx0 + 1, cw - 1);
+    const float *w3 = J.selW3 + c.ox;
+    uint8_t *roi = J.roi;
+    for (int oy = c.oy; oy < c.end; oy += 8) {
+        if (!c.active(J, oy) || w3[(size_t)oy * J.W] < 1e-4f)
+            continue;
+        const int cy0 = __ldg(J.ay.cbI0 + oy), cy1 = min(cy0 + 1, cyMax);
+        uint8_t *r0 = roi + (size_t)cy0 * cw, *r1 = roi + (size_t)cy1 * cw;
+        r0[cx0] = 1;
+        r0[cx1] = 1;
+        r1[cx0] = 1;
+        r1[cx1] = 1;
+    }
 }
 
-__global__ void k_blend(LGCR_STAGE_ARGS) {
+__global__ void __launch_bounds__(256, 8)
+k_blend(LGCR_STAGE_ARGS) {
     gridDependency();
     const int f = findFrame(tileStart, njobs, blockIdx.x);
     const FrameJob &J = jobs[f];
-    int ox, oy;
-    tile32x8(blockIdx.x - tileStart[f], J.W, ox, oy);
-    if (ox >= J.W || oy >= J.H)
+    const ColumnWalk c(J, blockIdx.x - tileStart[f]);
+    if (!c.valid)
         return;
-    const size_t o = (size_t)oy * J.W + ox;
-    // final sample: to the typed output when nothing follows the blend
-    auto finish = [&](float u, float v) {
-        if (J.blendStores) {
-            storeChroma(J, 1, ox, oy, u);
-            storeChroma(J, 2, ox, oy, v);
-        } else {
-            J.oU[o] = u;
-            J.oV[o] = v;
-        }
-    };
-    if (!activeOut(J, ox, oy)) {
-        if (J.blendStores)
-            finish(J.oU[o], J.oV[o]);
-        return;
-    }
+    const int ox = c.ox;
     const float lam = J.strength4;
     const bool compressed = J.sparse &&
         (unsigned long long)J.counters[kCntActiveOutput] * 2ull < (unsigned long long)J.W * J.H;
-    const int cx = __ldg(J.ax.cbI0 + ox), cy = __ldg(J.ay.cbI0 + oy);
-    const float cxf = __ldg(J.ax.cbF + ox), cyf = __ldg(J.ay.cbF + oy);
-    const float plainU = J.oU[o], plainV = J.oV[o];
-    if (compressed) {
-        const float w3 = lam * J.selW3[o];
-        float valueU = plainU + lam * J.gU[o];
-        float valueV = plainV + lam * J.gV[o];
-        if (w3 != 0.0f) {
-            const float luma = bilinearFast(J.Y, J.sw, J.sh, __ldg(J.ax.lbI0 + ox), __ldg(J.ax.lbF + ox),
-                                            __ldg(J.ay.lbI0 + oy), __ldg(J.ay.lbF + oy));
-            const LgfSample m = lgfAt(J, cx, cxf, cy, cyf);
-            const float au = m.ab.x, bu = m.ab.y, av = m.ab.z, bv = m.ab.w, cu = m.conf.x, cv = m.conf.y;
-            valueU += w3 * cu * (au * luma + bu - plainU);
-            valueV += w3 * cv * (av * luma + bv - plainV);
+    const int cx = __ldg(J.ax.cbI0 + ox), lx = __ldg(J.ax.lbI0 + ox);
+    const float cxf = __ldg(J.ax.cbF + ox), lxf = __ldg(J.ax.lbF + ox);
+    auto lumaAt = [&](int oy) {
+        return bilinearFast(J.Y, J.sw, J.sh, lx, lxf, __ldg(J.ay.lbI0 + oy), __ldg(J.ay.lbF + oy));
+    };
+    for (int oy = c.oy; oy < c.end; oy += 8) {
+        const size_t o = (size_t)oy * J.W + ox;
+        // final sample: to the typed output when nothing follows the blend
+        auto finish = [&](float u, float v) {
+            if (J.blendStores) {
+                storeChroma(J, 1, ox, oy, u);
+                storeChroma(J, 2, ox, oy, v);
+            } else {
+                J.oU[o] = u;
+                J.oV[o] = v;
+            }
+        };
+        if (!c.active(J, oy)) {
+            if (J.blendStores)
+                finish(J.oU[o], J.oV[o]);
+            continue;
         }
-        finish(valueU, valueV);
-        return;
+        const int cy = __ldg(J.ay.cbI0 + oy);
+        const float cyf = __ldg(J.ay.cbF + oy);
+        const float plainU = J.oU[o], plainV = J.oV[o];
+        if (compressed) {
+            const float w3 = lam * J.selW3[o];
+            float valueU = plainU + lam * J.gU[o];
+            float valueV = plainV + lam * J.gV[o];
+            if (w3 != 0.0f) {
+                const float luma = lumaAt(oy);
+                const LgfSample m = lgfAt(J, cx, cxf, cy, cyf);
+                const float au = m.ab.x, bu = m.ab.y, av = m.ab.z, bv = m.ab.w, cu = m.conf.x, cv = m.conf.y;
+                valueU += w3 * cu * (au * luma + bu - plainU);
+                valueV += w3 * cv * (av * luma + bv - plainV);
+            }
+            finish(valueU, valueV);
+            continue;
+        }
+        const float w2v = J.selW2[o] * lam;
+        const float w3v = J.selW3[o] * lam;
+        if (w2v < 1e-4f && w3v < 1e-4f) {
+            if (J.blendStores)
+                finish(plainU, plainV);
+            continue;
+        }
+        const float L0 = lumaAt(oy);
+        const LgfSample m = lgfAt(J, cx, cxf, cy, cyf);
+        const float au = m.ab.x, bu = m.ab.y, av = m.ab.z, bv = m.ab.w, cu = m.conf.x, cv = m.conf.y;
+        finish(plainU + (w2v * (J.gU[o] - plainU) + w3v * cu * (au * L0 + bu - plainU)),
+               plainV + (w2v * (J.gV[o] - plainV) + w3v * cv * (av * L0 + bv - plainV)));
     }
-    const float w2v = J.selW2[o] * lam;
-    const float w3v = J.selW3[o] * lam;
-    if (w2v < 1e-4f && w3v < 1e-4f) {
-        if (J.blendStores)
-            finish(plainU, plainV);
-        return;
-    }
-    const float L0 = bilinearFast(J.Y, J.sw, J.sh, __ldg(J.ax.lbI0 + ox), __ldg(J.ax.lbF + ox),
-                                  __ldg(J.ay.lbI0 + oy), __ldg(J.ay.lbF + oy));
-    const LgfSample m = lgfAt(J, cx, cxf, cy, cyf);
-    const float au = m.ab.x, bu = m.ab.y, av = m.ab.z, bv = m.ab.w, cu = m.conf.x, cv = m.conf.y;
-    finish(plainU + (w2v * (J.gU[o] - plainU) + w3v * cu * (au * L0 + bu - plainU)),
-           plainV + (w2v * (J.gV[o] - plainV) + w3v * cv * (av * L0 + bv - plainV)));
 }
 
 } // namespace lgcr_b200

@@ -1054,7 +1054,7 @@ static int stageTilesShaped(const FrameJob &J, int s) {
     case S_DET_TRANSFER: return (J.guided && J.algo == 6 && !J.xferListed) ? cdiv(J.W, 32) * cdiv(J.H, 8) : 0;
     case S_DET_XFER_LIST: return J.xferListed ? 1 : 0;
     case S_ROI:
-    case S_BLEND: return (J.guided && J.algo == 4 && J.lgfRoiOnly) ? cdiv(J.W, 32) * cdiv(J.H, 8) : 0;
+    case S_BLEND: return (J.guided && J.algo == 4 && J.lgfRoiOnly) ? cdiv(J.W, 32) * cdiv(J.H, J.plainRows) : 0;
     case S_BM_GROUP: return J.bm ? cdiv(J.bmAnchorsX * J.bmAnchorsY, 8) : 0;
     case S_BM_AGG: return J.bm ? cdiv(J.W, 32) * cdiv(J.H, 8) : 0;
     case S_BP: return J.needBackProject ? cdiv(J.cw, 32) * cdiv(J.ch, 8) : 0;
