@@ -23,7 +23,8 @@
 //    Newton step needs no sign flips;
 //  * the bump term is evaluated for the columns that have a rescue weight
 //    (left-sited 4:2:0 and 4:2:2 columns 2p + 1 lie half a sample off and have
-//    none: the term was multiplied by zero there);
+//    none: the term was multiplied by zero there), or a direction that is not
+//    finite (NaN or overflowing float luma), whose bump times zero is NaN;
 //  * the sum of |w| of the fallback test is not accumulated: it is bounded by
 //    the kernel's own negative weight, and a pair that the bound does not
 //    clear is evaluated again with the sum.
@@ -132,6 +133,7 @@ struct Pair {
     int tx0, ty0;                 // common window
     int kind;                     // row of the pair weight table
     uint32_t bits, my;            // active taps of both columns, active rows
+    bool bump;                    // column 2p + 1 takes the bump term
 };
 
 struct PairAcc {
@@ -139,8 +141,8 @@ struct PairAcc {
 };
 
 // Pass 2 (recon.cpp:606-623): w = sim * (wbase + rescue * bump) over the
-// active taps, accumulated in FP64 in tap order. BOTH: both columns carry a
-// rescue weight, else only column 2p may. RADIAL: base weights are the pair's
+// active taps, accumulated in FP64 in tap order. BOTH: both columns take the
+// bump term, else only column 2p. RADIAL: base weights are the pair's
 // rows of the jinc phase table (rad), else wx(i) * wy(j). FULL: every column
 // but the first and last of the window is active for both pixels (all windows
 // away from the frame's sides), so only those two are tested.
@@ -236,8 +238,8 @@ __device__ __forceinline__ bool innerColumnsActive(uint32_t bits) {
 template <int UC, bool RADIAL>
 __device__ __forceinline__ void pairTapsFor(const FrameJob &J, const Pair &c, int oy,
                                             const float2 *rad, PairAcc &acc) {
-    // one variant per warp: lanes without a second rescue weight lose nothing in BOTH
-    const bool both = __any_sync(__activemask(), c.rescue[1] != 0.0f);
+    // one variant per warp: lanes without a second bump term lose nothing in BOTH
+    const bool both = __any_sync(__activemask(), c.bump);
     if (!innerColumnsActive<UC>(c.bits))
         pairTaps<UC, true, RADIAL, false, false>(J, c, oy, rad, acc);
     else if (both)
@@ -628,6 +630,8 @@ struct PairWork {
             g2p[q] = b.z;
             c.invG2Par[q] = fabsf(b.z);
         }
+        c.bump = on[1] && !(c.rescue[1] == 0.0f && fabsf(c.nx[1]) <= 2.0f && fabsf(c.ny[1]) <= 2.0f &&
+                            c.invG2Par[1] >= 0.0f);
         const float2 *rad = nullptr;
         if (RADIAL)
             rad = J.pairRad + ((size_t)__ldg(J.rad.yPhase + oy) * J.pairPhases + __ldg(J.pairPhase + p)) *
