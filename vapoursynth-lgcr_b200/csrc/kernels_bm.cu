@@ -12,6 +12,7 @@
 //                   stored to the typed output (the last stage)
 //                                               src/algos.cpp:663-677
 #include "kernels.cuh"
+#include "bm_rank.h"
 
 namespace lgcr_b200 {
 
@@ -88,7 +89,7 @@ k_bm_group(LGCR_STAGE_ARGS) {
     const int ax = __ldg(J.bmStartsX + anchor % J.bmAnchorsX);
     const float *U = J.oU, *V = J.oV;
     // candidate grid: dy outer, dx inner, steps of 4 over [-8, 8]
-    if (lane < 25) {
+    if (lane < kBmCandidates) {
         const int dy = -8 + 4 * (lane / 5), dx = -8 + 4 * (lane % 5);
         const int bx = iclamp(ax + dx, 0, W - kPatch), by = iclamp(ay + dy, 0, H - kPatch);
         cbx[warp][lane] = bx;
@@ -119,7 +120,7 @@ k_bm_group(LGCR_STAGE_ARGS) {
     bool keep = false;
     float myCost = 0.0f;
     int myBx = 0, myBy = 0;
-    if (lane < 25) {
+    if (lane < kBmCandidates) {
         myBx = cbx[warp][lane];
         myBy = cby[warp][lane];
         myCost = costs[warp][lane];
@@ -132,14 +133,7 @@ k_bm_group(LGCR_STAGE_ARGS) {
     }
     const unsigned kept = __ballot_sync(0xffffffffu, keep);
     if (keep) {
-        int rank = 0;
-        for (int d = 0; d < 25; ++d) {
-            if (d == lane || !((kept >> d) & 1u))
-                continue;
-            const float cd = costs[warp][d];
-            if (cd < myCost || (cd == myCost && d < lane))
-                ++rank;
-        }
+        const int rank = keptRank(costs[warp], kept, lane);
         if (rank < kGroup) {
             bestC[warp][rank] = myCost;
             bestX[warp][rank] = myBx;
