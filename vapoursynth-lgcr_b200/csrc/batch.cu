@@ -50,6 +50,10 @@ struct lgcr_batch {
     size_t prefixCapacity = 0;
     DescriptorSlot slots[kDescriptorSlots];
     int next = 0;                       // slot of the next run
+    // scratch of the column-pair guided pass, one for all runs: a run waits on
+    // its stream for the last one that used it (pairsSlot, -1: none yet)
+    PairScratch pairs;
+    int pairsSlot = -1;
     int lastLaunches = 0;
     // profiling
     bool profiling = false;
@@ -142,14 +146,12 @@ struct GroupedPlan {
     std::vector<size_t> offset;         // groups + 1
 };
 
+// Frame ranges of the groups, and the work split of their launches.
 // groupMode: -1 upscaling frames alone, 0 one group, n >= 1 every n frames
-void planGroups(std::vector<FrameJob> &jobs, GroupedPlan &gp, int groupMode,
-                const LaunchConfig *cfg) {
+void formGroups(std::vector<FrameJob> &jobs, GroupedPlan &gp, int groupMode) {
     const int n = int(jobs.size());
     const int g = groupMode;
     gp.start.clear();
-    gp.plans.clear();
-    gp.offset.assign(1, 0);
     if (g >= 0) {
         for (int f = 0; f < n; f += (g > 0 ? g : n))
             gp.start.push_back(f);
@@ -162,10 +164,48 @@ void planGroups(std::vector<FrameJob> &jobs, GroupedPlan &gp, int groupMode,
                 gp.start.push_back(f);
     }
     gp.start.push_back(n);
+    for (size_t k = 0; k + 1 < gp.start.size(); ++k)
+        shapeJobs(jobs.data() + gp.start[k], gp.start[k + 1] - gp.start[k]);
+}
+
+// All earlier runs have ended.
+void waitRuns(lgcr_batch *b) {
+    for (auto &sl : b->slots)
+        if (sl.pending)
+            cudaEventSynchronize(sl.done);
+}
+
+// Scratch of the groups' column-pair launches, which run one after another.
+// Returns what a captured graph depends on: the launches that take pairs.
+std::string attachPairs(lgcr_batch *b, std::vector<FrameJob> &jobs, const GroupedPlan &gp, cudaStream_t s) {
+    size_t need = 0;
+    for (size_t k = 0; k + 1 < gp.start.size(); ++k)
+        need = std::max(need, PairScratch::bytesFor(jobs.data() + gp.start[k], gp.start[k + 1] - gp.start[k]));
+    if (need > b->pairs.bytes) {
+        waitRuns(b);
+        b->pairs.reserve(need);
+    } else if (need > 0 && b->pairsSlot >= 0) {
+        cudaStreamWaitEvent(s, b->slots[b->pairsSlot].done, 0);
+    }
+    std::string sig;
+    for (size_t k = 0; k + 1 < gp.start.size(); ++k) {
+        b->pairs.attach(jobs.data() + gp.start[k], gp.start[k + 1] - gp.start[k]);
+        int chunk = 0;
+        for (int f = gp.start[k]; f < gp.start[k + 1]; ++f)
+            if (jobs[f].pairSup > 0)
+                chunk = jobs[f].pairChunk;
+        sig += "|p" + std::to_string(chunk);
+    }
+    if (need > 0)
+        b->pairsSlot = b->next;
+    return sig;
+}
+
+void planGroups(const std::vector<FrameJob> &jobs, GroupedPlan &gp, const LaunchConfig *cfg) {
     const int groups = int(gp.start.size()) - 1;
     gp.plans.resize(groups);
+    gp.offset.assign(1, 0);
     for (int k = 0; k < groups; ++k) {
-        shapeJobs(jobs.data() + gp.start[k], gp.start[k + 1] - gp.start[k]);
         const std::vector<FrameJob> sub(jobs.begin() + gp.start[k], jobs.begin() + gp.start[k + 1]);
         planStages(sub, gp.plans[k], cfg);
         gp.offset.push_back(gp.offset.back() + gp.plans[k].prefix.size());
@@ -286,6 +326,13 @@ int lgcr_batch_run(lgcr_batch *b, const lgcr_batch_item *items, int count, void 
             return LGCR_E_NOMEM;
         }
         Workspace *ws = F->acquire(false);
+        if (!ws && b->pairs.base) {
+            // the pair form's scratch may be what the workspace lacks
+            waitRuns(b);
+            b->pairs.release();
+            cudaGetLastError();
+            ws = F->acquire(false);
+        }
         if (!ws) {
             giveBack();
             setError("LGCR: device workspace allocation failed");
@@ -309,8 +356,9 @@ int lgcr_batch_run(lgcr_batch *b, const lgcr_batch_item *items, int count, void 
         sig += buf;
     }
     GroupedPlan plan;
-    planGroups(jobs, plan, b->groupMode >= -1 ? b->groupMode : batchGroupFrames(),
-               b->ownConfig ? &b->cfg : nullptr);
+    formGroups(jobs, plan, b->groupMode >= -1 ? b->groupMode : batchGroupFrames());
+    sig += attachPairs(b, jobs, plan, s);
+    planGroups(jobs, plan, b->ownConfig ? &b->cfg : nullptr);
     std::memcpy(sl.hJobs, jobs.data(), sizeof(FrameJob) * count);
     for (size_t k = 0; k < plan.plans.size(); ++k)
         std::memcpy(sl.hPrefix + plan.offset[k], plan.plans[k].prefix.data(),

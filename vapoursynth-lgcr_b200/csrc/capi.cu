@@ -203,6 +203,8 @@ int lgcr_recon_frame(lgcr_recon *h, const lgcr_plane in[3], const lgcr_plane out
     if (e == cudaSuccess) {
         buildJob(t, *ws->hJob);
         shapeJobs(ws->hJob, 1);
+        ws->pairs.reserve(PairScratch::bytesFor(ws->hJob, 1));
+        ws->pairs.attach(ws->hJob, 1);
         e = cudaMemcpyAsync(ws->dJob, ws->hJob, sizeof(FrameJob), cudaMemcpyHostToDevice, s);
     }
     if (e == cudaSuccess) {

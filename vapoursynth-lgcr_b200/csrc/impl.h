@@ -91,6 +91,34 @@ struct DeviceTables {
 
 struct Filter;
 
+// Device scratch of the guided pass by column pairs: what its kernels hand on
+// per listed pixel (contexts, 32 bytes; jinc frames: window extrema, 24). One
+// launch of frames shares it, and a launch with more list entries than it holds
+// goes through it in chunks, so it stays below kMost entries (64 bytes each,
+// jinc 112: 512 or 896 MB) whatever the number of the frames. Each chunk costs
+// the ends of its kernels: with 1, 2 and 4 million entries and without a limit,
+// one 1080p -> 4K 16-bit jinc frame (4.1 million) takes 1873, 1812, 1786 and
+// 1777 us, 64 640x360 frames (7.4 million) 2708, 2616, 2590 and 2559 us, and 8
+// 1080p + 8 4K guided frames beside as many of detail transfer (41 million)
+// 16.65, 16.30, 16.16 and 16.16 ms.
+struct PairScratch {
+    static constexpr long long kMost = 8 << 20;
+    void *base = nullptr;
+    size_t bytes = 0;
+    PairScratch() = default;
+    PairScratch(const PairScratch &) = delete;
+    PairScratch &operator=(const PairScratch &) = delete;
+    ~PairScratch() { release(); }
+    // What the launch of these shaped jobs takes (0: no frame takes pairs).
+    static size_t bytesFor(const FrameJob *jobs, int n);
+    // Grows to `need` bytes. Work that uses the scratch must have ended.
+    bool reserve(size_t need);
+    // Gives the jobs of one launch the scratch; where it could not be had they
+    // take the pixel form, which needs none.
+    void attach(FrameJob *jobs, int n) const;
+    void release();
+};
+
 // Per-frame device workspace (planes sized for the filter's geometry).
 struct Workspace {
     Filter *owner = nullptr;
@@ -105,7 +133,7 @@ struct Workspace {
     double *uvd = nullptr;
     float *hTab = nullptr;
     float *wExt = nullptr;              // W x H float4 hull plane, then W x H float2 luma plane
-    float *context = nullptr;           // guided pixel contexts (in hTab's region where that is free)
+    PairScratch pairs;                  // per-frame form (a batch has its own)
     uint32_t *actList = nullptr;
     uint32_t *chromaList = nullptr;
     float *aff = nullptr, *yc1 = nullptr, *yc2 = nullptr, *ycTmp = nullptr;
@@ -177,7 +205,8 @@ void buildJob(const FrameTask &t, FrameJob &job);
 
 // Work split of the map and plain stages for the frames of one launch (call
 // once for the jobs that are planned and launched together, before they are
-// copied to the device).
+// copied to the device). Frames whose guided pass takes column pairs
+// (pairSup > 0) then need a PairScratch.
 void shapeJobs(FrameJob *jobs, int n);
 
 // Stage scheduler: launches every stage once over all jobs. `dJobs` is the

@@ -79,10 +79,11 @@ __global__ void k_guided_staged_r(LGCR_STAGE_ARGS);
 __global__ void k_guided_o(LGCR_STAGE_ARGS);
 __global__ void k_guided3_o(LGCR_STAGE_ARGS);
 __global__ void k_guided_staged_o(LGCR_STAGE_ARGS);
-__global__ void k_pair_extrema(LGCR_STAGE_ARGS);
-__global__ void k_guide_setup(LGCR_STAGE_ARGS);
-__global__ void k_guided_pair(LGCR_STAGE_ARGS);
-__global__ void k_guided_pair_r(LGCR_STAGE_ARGS);
+// `first`: list entry (over the launch's concatenated lists) the chunk starts at
+__global__ void k_pair_extrema(LGCR_STAGE_ARGS, unsigned long long first);
+__global__ void k_guide_setup(LGCR_STAGE_ARGS, unsigned long long first);
+__global__ void k_guided_pair(LGCR_STAGE_ARGS, unsigned long long first);
+__global__ void k_guided_pair_r(LGCR_STAGE_ARGS, unsigned long long first);
 // dynamic shared memory of k_guided_staged: 8 warps x 8 x 40 samples of
 // lc (4 B) and the (u, v) pair (16 B)
 constexpr size_t kGuidedStageBytes = size_t(8) * 8 * 40 * (4 + 16);

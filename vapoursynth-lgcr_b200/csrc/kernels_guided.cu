@@ -113,7 +113,7 @@ __device__ __forceinline__ void divide2(double n0, double n1, double d, double &
 }
 
 // Context of one listed pixel (k_guide_setup to k_guided_pair): two float4 at
-// list index 2 * entry + column.
+// 2 * (entry's place in the chunk) + column.
 //   a = (L0, nx, ny, 1/sigma^2), the last negative when a similarity
 //       denominator may reach 2^64
 //   b = (fade, rescue, 1/(g * aniso)^2, ssRamp), the third negative when the
@@ -425,7 +425,7 @@ __device__ __forceinline__ void pairColumns(const FrameJob &J, uint32_t e, int &
 struct ExtremaWork {
     static __device__ __forceinline__ bool mine(const FrameJob &J) { return J.pairSup > 0 && J.radial; }
     static constexpr int kPer = 1;                       // threads per list entry
-    static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx) {
+    static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx, unsigned slot) {
         int ox, oy;
         bool on[2];
         pairColumns(J, __ldg(J.actList + idx), ox, oy, on[0], on[1]);
@@ -471,8 +471,8 @@ struct ExtremaWork {
                 v1 = sclamp(v1, (double)(h.mnV[q] - J.margin), (double)(h.mxV[q] + J.margin));
             }
             const size_t o = (size_t)oy * J.W + ox + q;
-            J.wHull[o] = make_float4(h.mnU[q], h.mxU[q], h.mnV[q], h.mxV[q]);
-            J.wLum[o] = make_float2(h.mnL[q], h.mxL[q]);
+            J.pairHull[2 * slot + q] = make_float4(h.mnU[q], h.mxU[q], h.mnV[q], h.mxV[q]);
+            J.pairLum[2 * slot + q] = make_float2(h.mnL[q], h.mxL[q]);
             J.oU[o] = (float)v0;
             J.oV[o] = (float)v1;
         }
@@ -484,14 +484,14 @@ struct ExtremaWork {
 struct SetupWork {
     static __device__ __forceinline__ bool mine(const FrameJob &J) { return J.pairSup > 0; }
     static constexpr int kPer = 2;
-    static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx) {
+    static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx, unsigned slot) {
         const uint32_t e = __ldg(J.actList + (idx >> 1));
         const int ox = (int)(e & 0xfffeu) + (int)(idx & 1u), oy = (int)(e >> 16);
         if (ox >= J.W || ((e & 1u) && !pixelActive(J, ox, oy)))
             return;
         const AxisView &ax = J.ax, &ay = J.ay;
         const int sw = J.sw, sh = J.sh;
-        const float2 lum = J.wLum[(size_t)oy * J.W + ox];
+        const float2 lum = J.radial ? J.pairLum[slot] : J.wLum[(size_t)oy * J.W + ox];
         const float lx = __ldg(ax.lpos + ox), ly = __ldg(ay.lpos + oy);
         const float lcN = ldf(J.lc + (size_t)__ldg(ay.nearest + oy) * J.cw + __ldg(ax.nearest + ox));
         float mutualFade = 1.0f;
@@ -589,8 +589,8 @@ struct SetupWork {
         const float g2p = J.invGsigma2 / (aniso * aniso);
         // every tap's similarity denominator is at most this (see guidedPixel)
         const bool safe = (1.0f + m * m * invSigma2) < kRcpFastLimit;
-        J.context[2 * idx] = make_float4(L0, nx, ny, withSign(invSigma2, !safe));
-        J.context[2 * idx + 1] = make_float4(fade, rescue, withSign(g2p, !hasDir), ssRamp);
+        J.context[2 * slot] = make_float4(L0, nx, ny, withSign(invSigma2, !safe));
+        J.context[2 * slot + 1] = make_float4(fade, rescue, withSign(g2p, !hasDir), ssRamp);
     }
 };
 
@@ -601,7 +601,7 @@ struct PairWork {
         return J.pairSup > 0 && (J.radial != 0) == RADIAL;
     }
     static constexpr int kPer = 1;
-    static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx) {
+    static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx, unsigned slot) {
         int ox, oy;
         bool on[2];
         pairColumns(J, __ldg(J.actList + idx), ox, oy, on[0], on[1]);
@@ -621,7 +621,7 @@ struct PairWork {
         c.my = __ldg(J.ay.amBits + oy);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const float4 a = __ldg(J.context + 4 * idx + 2 * q), b = __ldg(J.context + 4 * idx + 2 * q + 1);
+            const float4 a = __ldg(J.context + 4 * slot + 2 * q), b = __ldg(J.context + 4 * slot + 2 * q + 1);
             c.L0[q] = a.x; c.nx[q] = a.y; c.ny[q] = a.z;
             safe[q] = __float_as_int(a.w) >= 0;
             c.invSigma2[q] = fabsf(a.w);
@@ -669,15 +669,16 @@ struct PairWork {
         }
         const size_t o = (size_t)oy * J.W + ox;
         float4 hull[2];
-        hull[0] = __ldg(J.wHull + o);
-        hull[1] = __ldg(J.wHull + o + (T.two ? 1 : 0));
+        const float4 *hulls = RADIAL ? J.pairHull + 2 * slot : J.wHull + o;
+        hull[0] = __ldg(hulls);
+        hull[1] = __ldg(hulls + (T.two ? 1 : 0));
         Acc sums[2];
         bool good[2];
         // TRecon: the neighbours' motion-compensated samples follow the spatial
         // taps in the same accumulators and extend the hull. Then the fallback test.
         auto close = [&](int q) {
             if (!RADIAL && J.tnbCount > 0 && on[q]) {
-                const float ssRamp = J.context[4 * idx + 2 * q + 1].w;
+                const float ssRamp = J.context[4 * slot + 2 * q + 1].w;
                 const float2 lum = __ldg(J.wLum + o + q);
                 const float m = smax(smax(0.0f, fabsf(lum.y - c.L0[q])), fabsf(lum.x - c.L0[q]));
                 const float sigLoc = smax(J.sigma, (J.sratio + (J.sdb - J.sratio) * ssRamp) * m);
@@ -742,7 +743,7 @@ struct PairWork {
             if ((RADIAL || J.algo != 2) && on[q]) {
                 Guided g;
                 g.u = valueU; g.v = valueV;
-                g.L0 = c.L0[q]; g.ssRamp = J.context[4 * idx + 2 * q + 1].w; g.guideFade = c.fade[q];
+                g.L0 = c.L0[q]; g.ssRamp = J.context[4 * slot + 2 * q + 1].w; g.guideFade = c.fade[q];
                 g.nx = c.nx[q]; g.ny = c.ny[q]; g.hasDir = __float_as_int(g2p[q]) >= 0;
                 g.havePlain = RADIAL;
                 g.plainU = g.plainV = 0.0f;
@@ -769,48 +770,60 @@ struct PairWork {
     }
 };
 
-// Persistent grid over the concatenated lists of the launch's frames: blocks
-// stride over them side by side, so the rows in flight stay close together in
-// L2 (one contiguous share per block measured 10 % slower on 4K frames). The
-// descriptor of the current frame is kept in shared memory.
+// Persistent grid over the entries [first, first + pairChunk) of the
+// concatenated lists of the launch's frames: blocks stride over them side by
+// side, so the rows in flight stay close together in L2 (one contiguous share
+// per block measured 10 % slower on 4K frames). The descriptor of the current
+// frame is kept in shared memory. An entry's place in the chunk, the same for
+// every kernel, is where the scratch holds its contexts and extrema.
 template <class Work>
-__device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int njobs) {
+__device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int njobs,
+                                         unsigned long long first) {
     __shared__ unsigned long long pre[kPairMaxFrames + 1];
     __shared__ FrameJob sJob;
+    __shared__ int sChunk;
     const int tid = threadIdx.x;
+    unsigned long long before = 0;                       // threads of the frames before this part
     for (int chunk = 0; chunk < njobs; chunk += kPairMaxFrames) {
         const int n = min(kPairMaxFrames, njobs - chunk);
         __syncthreads();
         for (int i = tid; i < n; i += kPairThreads) {
             const FrameJob &J = jobs[chunk + i];
-            pre[i + 1] = Work::mine(J) ? J.counters[kCntPairs] * Work::kPer : 0ull;
+            pre[i + 1] = J.pairSup > 0 ? J.counters[kCntPairs] * Work::kPer : 0ull;
+            if (J.pairSup > 0)
+                sChunk = J.pairChunk;                    // one value for all frames
         }
         __syncthreads();
         if (tid == 0) {
-            unsigned long long acc = 0;
-            pre[0] = 0ull;
+            unsigned long long acc = before;
+            pre[0] = before;
             for (int i = 1; i <= n; ++i)
                 pre[i] = acc += pre[i];
         }
         __syncthreads();
-        const unsigned long long total = pre[n];
+        const unsigned long long base = first * Work::kPer;
+        const unsigned long long begin = max(pre[0], base);
+        const unsigned long long total = before = pre[n];
+        const unsigned long long end = min(total, base + (unsigned long long)sChunk * Work::kPer);
         int staged = -1, f = 0;
-        for (unsigned long long lo = (unsigned long long)blockIdx.x * kPairThreads; lo < total;
+        for (unsigned long long lo = begin + (unsigned long long)blockIdx.x * kPairThreads; lo < end;
              lo += (unsigned long long)gridDim.x * kPairThreads) {
-            const unsigned long long hi = min(lo + kPairThreads, total);
+            const unsigned long long hi = min(lo + kPairThreads, end);
             while (pre[f + 1] <= lo)
                 ++f;
             for (int g = f; g < n && pre[g] < hi; ++g) {
                 if (pre[g + 1] == pre[g])
                     continue;
                 if (g != staged) {
+                    if (!Work::mine(jobs[chunk + g]))
+                        continue;
                     __syncthreads();
                     stageJob(jobs, chunk + g, sJob);
                     staged = g;
                 }
                 const unsigned long long w = lo + tid;
-                if (w >= pre[g] && w < pre[g + 1])
-                    Work::run(sJob, w - pre[g]);
+                if (w >= pre[g] && w < pre[g + 1] && w < hi)
+                    Work::run(sJob, w - pre[g], (unsigned)(w - base));
             }
         }
     }
@@ -819,31 +832,35 @@ __device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int 
 } // namespace
 
 __global__ void __launch_bounds__(kPairThreads, 5)
-k_pair_extrema(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+k_pair_extrema(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs,
+               unsigned long long first) {
     gridDependency();
     (void)tileStart;
-    pairGrid<ExtremaWork>(jobs, njobs);
+    pairGrid<ExtremaWork>(jobs, njobs, first);
 }
 
 __global__ void __launch_bounds__(kPairThreads, 8)
-k_guide_setup(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+k_guide_setup(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs,
+              unsigned long long first) {
     gridDependency();
     (void)tileStart;
-    pairGrid<SetupWork>(jobs, njobs);
+    pairGrid<SetupWork>(jobs, njobs, first);
 }
 
 __global__ void __launch_bounds__(kPairThreads, 4)
-k_guided_pair(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+k_guided_pair(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs,
+              unsigned long long first) {
     gridDependency();
     (void)tileStart;
-    pairGrid<PairWork<false>>(jobs, njobs);
+    pairGrid<PairWork<false>>(jobs, njobs, first);
 }
 
 __global__ void __launch_bounds__(kPairThreads, 6)
-k_guided_pair_r(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs) {
+k_guided_pair_r(const FrameJob *__restrict__ jobs, const int *__restrict__ tileStart, int njobs,
+                unsigned long long first) {
     gridDependency();
     (void)tileStart;
-    pairGrid<PairWork<true>>(jobs, njobs);
+    pairGrid<PairWork<true>>(jobs, njobs, first);
 }
 
 } // namespace lgcr_b200

@@ -579,7 +579,7 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
     // writes every pixel and nothing here is needed (EARLY instance only:
     // compiled into the common one, the test costs the separable frames'
     // plain pass 5 % through its register allocation)
-    if (EARLY && skipListed && !J.hTab && (!J.wHull || J.radial) && !J.finalInTransfer &&
+    if (EARLY && skipListed && !J.hTab && !J.wHull && !J.finalInTransfer &&
         J.counters[kCntActiveOutput] >= (unsigned long long)J.W * J.H)
         return;
     int syLo = 0, nRows = 0;
@@ -615,7 +615,7 @@ __device__ __forceinline__ void plainStage(const FrameJob *__restrict__ jobs,
     // active-pixel bits: listed pixels are skipped here (after folding their
     // guided windows' extrema); algo 6 pixels the detail transfer leaves
     // alone are stored final here
-    const bool foldExtrema = J.wHull && !J.radial;  // implies fused row tables
+    const bool foldExtrema = J.wHull != nullptr;    // implies fused row tables
     const bool needAct = skipListed || J.finalInTransfer || foldExtrema;
     const bool maskWords = needAct && J.sparse && J.sameSize;
     if (maskWords && tid < rowsHere)

@@ -557,18 +557,8 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
     Slot sLumaTmp = take(size_t(p.outW) * sh * 4, !sameSize && !p.k.radial);  // luma / detail resize
     Slot sCnt = take(kCntCount * sizeof(unsigned long long));
     const bool listed = guided && (p.algo == 2 || p.algo == 4);
-    // context planes of the column-pair guided pass (32 bytes per pixel) share
-    // the horizontal table's region: frames whose windows k_plain folds have no
-    // table, except the integer selector's
-    const bool pairable = listed && p.k.kernel != Kernel::Bilinear;
-    const size_t contextBytes = size_t((p.outW + 1) / 2) * 2 * p.outH * 32;    // whole pairs
-    const size_t tableBytes = p.k.radial ? 0 : size_t(p.outW) * ch * 32;
-    const bool tableKept = p.algo == 4 && !isFloat() && !p.k.radial;
-    Slot sUvd = take(C * 16);
-    Slot sHTab = take(std::max(tableBytes, pairable && !tableKept ? contextBytes : 0),
-                      !p.k.radial || pairable);
-    Slot sCtx = take(contextBytes, pairable && tableKept);
-    Slot sWExt = take(O * 24, pairable);
+    Slot sUvd = take(C * 16), sHTab = take(size_t(p.outW) * ch * 32, !p.k.radial);
+    Slot sWExt = take(O * 24, listed && !p.k.radial && p.k.kernel != Kernel::Bilinear);
     Slot sList = take(O * 4, listed || (guided && p.algo == 6 && p.sparse));
     Slot sCList = take(C * 4, guided && p.algo == 6 && p.sparse);
     const bool algo6 = guided && p.algo == 6, algo4 = guided && p.algo == 4;
@@ -607,8 +597,7 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
     ws->oU = F(sOU); ws->oV = F(sOV); ws->lumaTmp = F(sLumaTmp);
     ws->counters = (unsigned long long *)ar.at(sCnt.off);
     ws->uvd = sUvd.on ? (double *)ar.at(sUvd.off) : nullptr;
-    ws->hTab = p.k.radial ? nullptr : F(sHTab);
-    ws->context = tableKept ? F(sCtx) : pairable ? F(sHTab) : nullptr;
+    ws->hTab = F(sHTab);
     ws->wExt = F(sWExt);
     ws->actList = sList.on ? (uint32_t *)ar.at(sList.off) : nullptr;
     ws->chromaList = sCList.on ? (uint32_t *)ar.at(sCList.off) : nullptr;
@@ -791,11 +780,7 @@ void buildJob(const FrameTask &t, FrameJob &J) {
     J.plainRows = J.plainFused ? T.plainRows : kPlainRowsShort;
     J.wHull = nullptr;
     J.wLum = nullptr;
-    if (ws.wExt && J.radial) {
-        // filled by the pair form's first pass
-        J.wHull = reinterpret_cast<float4 *>(ws.wExt);
-        J.wLum = reinterpret_cast<float2 *>(ws.wExt + size_t(J.W) * J.H * 4);
-    } else if (ws.wExt && J.listed && J.plainFused && J.kernel != 0 && T.aySup <= 8) {
+    if (ws.wExt && J.listed && J.plainFused && J.kernel != 0 && T.aySup <= 8) {
         // k_plain folds the guided windows' extrema for the listed pixels from
         // its staged rows; the horizontal table is then only needed for the
         // integer algo 4 plain base the guided pass recomputes
@@ -818,11 +803,10 @@ void buildJob(const FrameTask &t, FrameJob &J) {
     // shapeJobs decides whether a launch does.
     J.pairSup = 0;
     J.guideOnGrid = J.sameSize && J.inKind != kF32;
-    if (T.pairSup > 0 && ws.context && J.listed && J.noClampX && J.noClampY && J.bumpRcpSafe && !J.cedge &&
+    if (T.pairSup > 0 && J.listed && J.noClampX && J.noClampY && J.bumpRcpSafe && !J.cedge &&
         T.axSup == T.aySup && (T.axSup == 4 || T.axSup == 6 || T.axSup == 8) &&
         (J.radial ? radialPlainFused(J) : J.wHull != nullptr)) {
         J.pairSup = T.pairSup;
-        J.context = reinterpret_cast<float4 *>(ws.context);
         J.pairStart = T.pairStart;
         J.pairBits = T.pairBits;
         J.pairKind = T.pairKind;
@@ -832,10 +816,6 @@ void buildJob(const FrameTask &t, FrameJob &J) {
         J.pairRad = reinterpret_cast<const float2 *>(T.pairRad);
         J.pairRadD = reinterpret_cast<const double2 *>(T.pairRadD);
         J.radSums = reinterpret_cast<const double2 *>(T.radSums);
-    }
-    if (J.radial && J.pairSup == 0) {
-        J.wHull = nullptr;
-        J.wLum = nullptr;
     }
     // algo 6
     J.aff = ws.aff; J.yc1 = ws.yc1; J.yc2 = ws.yc2;
@@ -1114,10 +1094,6 @@ void shapeJobs(FrameJob *jobs, int n) {
         if (J.pairSup == 0 || pixels[J.radial ? 1 : 0] >= (J.radial ? kPairPixelsJinc : kPairPixels))
             continue;
         J.pairSup = 0;
-        if (J.radial) {
-            J.wHull = nullptr;
-            J.wLum = nullptr;
-        }
     }
     const int plain = longest({kPlainRows, 32, 16, 8}, [](const FrameJob &J, int rows) {
         return (long long)cdiv(J.W, 32) * cdiv(J.H, rows);
@@ -1127,6 +1103,76 @@ void shapeJobs(FrameJob *jobs, int n) {
         jobs[f].markWords = mark;
         jobs[f].countChunk = count;
         jobs[f].plainRows = std::min(jobs[f].plainRows, plain);
+    }
+}
+
+// Entries and bytes of the scratch for the pairing frames of one launch (a
+// frame lists at most every pair of its columns).
+static void pairScratchSize(const FrameJob *jobs, int n, long long &entries, size_t &perEntry) {
+    entries = 0;
+    perEntry = 2 * 2 * sizeof(float4);
+    for (int f = 0; f < n; ++f)
+        if (jobs[f].pairSup > 0) {
+            entries += (long long)cdiv(jobs[f].W, 2) * jobs[f].H;
+            if (jobs[f].radial)
+                perEntry = 2 * (3 * sizeof(float4) + sizeof(float2));
+        }
+}
+
+static int pairChunkEntries(long long entries) {
+    return int((std::min(entries, PairScratch::kMost) + 127) / 128 * 128);
+}
+
+void PairScratch::release() {
+    if (base)
+        cudaFree(base);
+    base = nullptr;
+    bytes = 0;
+}
+
+size_t PairScratch::bytesFor(const FrameJob *jobs, int n) {
+    long long entries = 0;
+    size_t perEntry = 0;
+    pairScratchSize(jobs, n, entries, perEntry);
+    return size_t(pairChunkEntries(entries)) * perEntry;
+}
+
+bool PairScratch::reserve(size_t need) {
+    if (need <= bytes)
+        return true;
+    release();
+    if (cudaMalloc(&base, need) != cudaSuccess) {
+        cudaGetLastError();                            // not this call's error: it has another way
+        base = nullptr;
+        return false;
+    }
+    bytes = need;
+    // as for new workspaces (makeWorkspace)
+    if (const char *e = std::getenv("LGCR_POISON_WORKSPACE"); e && e[0] == '1')
+        cudaMemset(base, 0xFF, bytes);
+    return true;
+}
+
+void PairScratch::attach(FrameJob *jobs, int n) const {
+    long long entries = 0;
+    size_t perEntry = 0;
+    pairScratchSize(jobs, n, entries, perEntry);
+    const size_t chunk = pairChunkEntries(entries);
+    const bool have = base && chunk * perEntry <= bytes;
+    for (int f = 0; f < n; ++f) {
+        FrameJob &J = jobs[f];
+        if (J.pairSup == 0)
+            continue;
+        if (!have) {
+            J.pairSup = 0;
+            continue;
+        }
+        J.pairChunk = int(chunk);
+        J.context = static_cast<float4 *>(base);
+        if (J.radial) {
+            J.pairHull = J.context + 4 * chunk;
+            J.pairLum = reinterpret_cast<float2 *>(J.pairHull + 2 * chunk);
+        }
     }
 }
 
@@ -1207,24 +1253,32 @@ int launchStages(const std::vector<FrameJob> &jobs, const StagePlan &plan, const
             (J.pairSup == 0 ? single : J.radial ? pairsRadial : pairs) = true;
     if (plan.totals[S_GUIDED] > 0 && (pairs || pairsRadial)) {
         // persistent grids over the pair lists
-        using PairKernel = void (*)(const FrameJob *, const int *, int);
+        using PairKernel = void (*)(const FrameJob *, const int *, int, unsigned long long);
         static const PairKernel kernels[4] = {k_pair_extrema, k_guide_setup, k_guided_pair,
                                               k_guided_pair_r};
         static int gridBlocks[4] = {0, 0, 0, 0};
         const bool run[4] = {pairsRadial, true, pairs, pairsRadial};
-        for (int k = 0; k < 4; ++k) {
-            if (!run[k])
-                continue;
-            if (gridBlocks[k] == 0) {
-                int dev = 0, sms = 0, perSm = 0;
-                cudaGetDevice(&dev);
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernels[k], 128, 0);
-                gridBlocks[k] = std::max(1, sms * std::max(1, perSm));
+        long long entries = 0, chunk = 0;
+        size_t perEntry = 0;
+        pairScratchSize(jobs.data(), n, entries, perEntry);
+        for (const FrameJob &J : jobs)
+            if (J.pairSup > 0)
+                chunk = J.pairChunk;
+        for (long long first = 0; first < entries; first += chunk)
+            for (int k = 0; k < 4; ++k) {
+                if (!run[k])
+                    continue;
+                if (gridBlocks[k] == 0) {
+                    int dev = 0, sms = 0, perSm = 0;
+                    cudaGetDevice(&dev);
+                    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernels[k], 128, 0);
+                    gridBlocks[k] = std::max(1, sms * std::max(1, perSm));
+                }
+                launchAfter(kernels[k], dim3(gridBlocks[k]), dim3(128), 0, stream, dJobs, pre(S_GUIDED), n,
+                            (unsigned long long)first);
+                ++launches;
             }
-            launchAfter(kernels[k], dim3(gridBlocks[k]), dim3(128), 0, stream, dJobs, pre(S_GUIDED), n);
-            ++launches;
-        }
     }
     if (plan.totals[S_GUIDED] > 0 && single) {
         // persistent grid: enough resident blocks to fill every SM

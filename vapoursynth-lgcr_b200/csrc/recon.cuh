@@ -133,7 +133,12 @@ struct __align__(16) FrameJob {
     // guided pass by column pairs (kernels_guided.cu): pairSup > 0 and the work
     // list holds pairs (y << 16 | even x | 1 when only one column is active)
     int pairSup;                       // samples of a pair's common window
+    // scratch of the launch (PairScratch), entry by entry of the part of the
+    // concatenated lists that a chunk of launches covers
+    int pairChunk;                     // list entries of a chunk
     float4 *context;                   // two per listed pixel: k_guide_setup's result
+    float4 *pairHull;                  // jinc frames: window chroma hull per listed pixel (as wHull)
+    float2 *pairLum;                   // jinc frames: window luma extrema per listed pixel (as wLum)
     int guideOnGrid;                   // guide positions are luma samples (same size, integer)
     const int *pairStart;              // per pair: first sample of the window
     const uint32_t *pairBits;          // per pair: active taps (low half even, high half odd column)

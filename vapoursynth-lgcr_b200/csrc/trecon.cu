@@ -354,6 +354,8 @@ int lgcr_trecon_frame(lgcr_trecon *t, const lgcr_plane cur[3], const lgcr_plane 
     FrameJob &J = *ws->hJob;
     buildJob(task, J);
     shapeJobs(&J, 1);
+    ws->pairs.reserve(PairScratch::bytesFor(&J, 1));
+    ws->pairs.attach(&J, 1);
     J.lumaNormalize = F.isFloat() ? 1 : 0;
     J.gateDense = 1;
     J.shiftXd = task.p.shiftX;
