@@ -6,6 +6,9 @@
 // the device (k_bm_group) and for the host's sweep of cost patterns.
 #pragma once
 
+#include <cstdint>
+#include <cstring>
+
 #ifdef __CUDACC__
 #define LGCR_HOST_DEVICE __host__ __device__ __forceinline__
 #else
@@ -16,17 +19,19 @@ namespace lgcr_b200 {
 
 constexpr int kBmCandidates = 25;
 
+// A cost is a mean of squares, so it is not below zero and its bits order as
+// its value; those of a NaN lie above infinity's.
+LGCR_HOST_DEVICE uint32_t costBits(float c) {
+    uint32_t b;
+    memcpy(&b, &c, sizeof(b));
+    return b & 0x7fffffffu;
+}
+
 LGCR_HOST_DEVICE int keptRank(const float *costs, unsigned kept, int me) {
-    const float mine = costs[me];
-    const bool last = mine != mine;
+    const uint32_t mine = costBits(costs[me]);
     int rank = 0;
-    for (int d = 0; d < kBmCandidates; ++d) {
-        if (d == me || !((kept >> d) & 1u))
-            continue;
-        const float c = costs[d];
-        if (last ? (c == c || d < me) : (c < mine || (c == mine && d < me)))
-            ++rank;
-    }
+    for (int d = 0; d < kBmCandidates; ++d)              // an earlier one of equal cost goes first
+        rank += int((kept >> d) & 1u & unsigned(costBits(costs[d]) < mine + (d < me ? 1u : 0u)));
     return rank;
 }
 
