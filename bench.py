@@ -280,6 +280,23 @@ def reference_scene_420ps(width=1920, height=1080):
     return y, box(u), box(v)
 
 
+def cpu_baseline(frames, specs):
+    """The workload on the reference's AVX2 build on this host's cores. That
+    build is made from the reference's sources; without it the device figures
+    still stand."""
+    from oracle import oracle as O
+    if not O.available("avx2"):
+        return {"unavailable": f"no reference AVX2 build in {os.path.relpath(O.LIBDIR, os.path.dirname(os.path.abspath(__file__)))}"}
+    threads = cpu_threads()
+    value, total_s, times = run_cpu(frames, specs, 1, 0, threads, threads, min_seconds=10.0)
+    return {"value": round(value, 3), "unit": "Mpix/s", "cores": threads, "kind": "reference",
+            "sample": f"{len(times)} rounds of {threads} frames (alternating 1080p/4K, algo 2/6, "
+                      f"one frame per thread) from the workload, reference AVX2 build "
+                      f"(oracle/_ref), {total_s:.1f} s",
+            **host_cpu(),
+            "reference_scene": reference_scene_fps()}
+
+
 def reference_scene_fps(seconds=3.0):
     """Single-thread time per frame of the reference's AVX2 build on its own
     benchmark scene at 1080p, algo 2, lanczos3, sparse, beside the published
@@ -1244,21 +1261,7 @@ def our_arm(args):
             made = pool.map(_gen_serve, [(k, 7000 + 97 * k + s) for k, s in keys])
         result["serving"] = serving_leg(dict(zip(keys, made)), args.serve_requests, lanes=args.serve_lanes)
     if rank == 0 and cpu_frames is not None:
-        # the reference's CPU build is made from its sources; without it the
-        # device figures still stand
-        try:
-            threads = cpu_threads()
-            value_cpu, total_s, times = run_cpu(cpu_frames, specs, 1, 0, threads, threads,
-                                                min_seconds=10.0)
-            result["cpu_baseline"] = {
-                "value": round(value_cpu, 3), "unit": "Mpix/s", "cores": threads, "kind": "reference",
-                "sample": f"{len(times)} rounds of {threads} frames (alternating 1080p/4K, algo 2/6, "
-                          f"one frame per thread) from the workload, reference AVX2 build "
-                          f"(oracle/_ref), {total_s:.1f} s",
-                **host_cpu(),
-                "reference_scene": reference_scene_fps()}
-        except FileNotFoundError as e:
-            result["cpu_baseline"] = {"unavailable": str(e).split(":")[0]}
+        result["cpu_baseline"] = cpu_baseline(cpu_frames, specs)
     if world > 1:
         torch.distributed.barrier()
         torch.distributed.destroy_process_group()
