@@ -159,7 +159,7 @@ int lgcr_recon_frame(lgcr_recon *h, const lgcr_plane in[3], const lgcr_plane out
         setError("LGCR: failed to upload geometry tables");
         return LGCR_E_NOMEM;
     }
-    Workspace *ws = F.acquire();
+    Workspace *ws = F.acquire(true, &t);
     if (!ws) {
         setError("LGCR: device workspace allocation failed");
         return LGCR_E_NOMEM;

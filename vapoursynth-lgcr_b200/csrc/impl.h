@@ -105,6 +105,7 @@ struct PairScratch {
     static constexpr long long kMost = 8 << 20;
     void *base = nullptr;
     size_t bytes = 0;
+    bool owned = false;                 // else part of a workspace's arena
     PairScratch() = default;
     PairScratch(const PairScratch &) = delete;
     PairScratch &operator=(const PairScratch &) = delete;
@@ -179,9 +180,11 @@ struct Filter {
     // A workspace from the filter's pool (per-frame form: with host staging;
     // batched/serving forms: without). The caller must order its work after
     // the workspace's previous frame (event `done`) when `used` is set.
-    Workspace *acquire(bool hostStaging = true);
+    // `task` (its planes and workspace not used): the frame that a new workspace
+    // of the per-frame form is made for; its pair scratch then comes with it.
+    Workspace *acquire(bool hostStaging, const FrameTask *task = nullptr);
     void release(Workspace *ws);
-    std::unique_ptr<Workspace> makeWorkspace(bool hostStaging);
+    std::unique_ptr<Workspace> makeWorkspace(bool hostStaging, size_t pairBytes);
     size_t workspaceBytes();
     FilterParams sited(int chromaLocation) const;
     bool isFloat() const { return fmt.sample_type == LGCR_ST_FLOAT; }

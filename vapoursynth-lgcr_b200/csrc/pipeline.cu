@@ -535,7 +535,21 @@ const DeviceTables *Filter::tablesFor(double shiftX, double shiftY) {
 // ---------------------------------------------------------------------------
 // workspaces
 // ---------------------------------------------------------------------------
-std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
+// Scratch of the column pairs of one frame alone, before it has a workspace.
+static size_t pairBytesAlone(const FrameTask &task) {
+    Workspace planes;                   // whether a plane is there is all that counts
+    planes.hTab = planes.wExt = reinterpret_cast<float *>(sizeof(float4));
+    FrameTask t = task;
+    t.ws = &planes;
+    for (int i = 0; i < 3; ++i)
+        t.in[i] = t.out[i] = lgcr_plane{};
+    FrameJob J;
+    buildJob(t, J);
+    shapeJobs(&J, 1);
+    return PairScratch::bytesFor(&J, 1);
+}
+
+std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging, size_t pairBytes) {
     auto ws = std::make_unique<Workspace>();
     ws->owner = this;
     DeviceArena &ar = ws->arena;
@@ -557,7 +571,14 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
     Slot sLumaTmp = take(size_t(p.outW) * sh * 4, !sameSize && !p.k.radial);  // luma / detail resize
     Slot sCnt = take(kCntCount * sizeof(unsigned long long));
     const bool listed = guided && (p.algo == 2 || p.algo == 4);
-    Slot sUvd = take(C * 16), sHTab = take(size_t(p.outW) * ch * 32, !p.k.radial);
+    // frames that take pairs have no horizontal table, except the integer
+    // selector's: the scratch then takes the table's place
+    const size_t tableBytes = p.k.radial ? 0 : size_t(p.outW) * ch * 32;
+    const bool tableKept = p.algo == 4 && !isFloat() && !p.k.radial;
+    Slot sUvd = take(C * 16);
+    Slot sHTab = take(tableKept ? tableBytes : std::max(tableBytes, pairBytes),
+                      !p.k.radial || pairBytes > 0);
+    Slot sPairs = tableKept ? take(pairBytes, pairBytes > 0) : sHTab;
     Slot sWExt = take(O * 24, listed && !p.k.radial && p.k.kernel != Kernel::Bilinear);
     Slot sList = take(O * 4, listed || (guided && p.algo == 6 && p.sparse));
     Slot sCList = take(C * 4, guided && p.algo == 6 && p.sparse);
@@ -597,8 +618,12 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
     ws->oU = F(sOU); ws->oV = F(sOV); ws->lumaTmp = F(sLumaTmp);
     ws->counters = (unsigned long long *)ar.at(sCnt.off);
     ws->uvd = sUvd.on ? (double *)ar.at(sUvd.off) : nullptr;
-    ws->hTab = F(sHTab);
+    ws->hTab = p.k.radial ? nullptr : F(sHTab);
     ws->wExt = F(sWExt);
+    if (pairBytes > 0) {
+        ws->pairs.base = ar.at(sPairs.off);
+        ws->pairs.bytes = pairBytes;
+    }
     ws->actList = sList.on ? (uint32_t *)ar.at(sList.off) : nullptr;
     ws->chromaList = sCList.on ? (uint32_t *)ar.at(sCList.off) : nullptr;
     ws->aff = F(sAff); ws->yc1 = F(sYc1); ws->yc2 = F(sYc2);
@@ -625,7 +650,7 @@ std::unique_ptr<Workspace> Filter::makeWorkspace(bool hostStaging) {
 
 // Prefer an idle workspace whose last frame has finished on the device; grow
 // the pool (up to a few per filter) rather than wait for one in flight.
-Workspace *Filter::acquire(bool hostStaging) {
+Workspace *Filter::acquire(bool hostStaging, const FrameTask *task) {
     constexpr int kMaxWorkspaces = 4;
     auto &pool = hostStaging ? idle : idleBatch;
     auto &count = hostStaging ? live : liveBatch;
@@ -645,7 +670,14 @@ Workspace *Filter::acquire(bool hostStaging) {
             return ws;   // caller orders its work after the event
         }
     }
-    auto ws = makeWorkspace(hostStaging);
+    // one allocation for both where there is room: a filter's first frame does
+    // not wait for a second one
+    const size_t pairBytes = task ? pairBytesAlone(*task) : 0;
+    auto ws = makeWorkspace(hostStaging, pairBytes);
+    if (!ws && pairBytes > 0) {
+        cudaGetLastError();
+        ws = makeWorkspace(hostStaging, 0);
+    }
     if (ws) {
         ws->hostStaging = hostStaging;
         count.fetch_add(1);
@@ -1124,10 +1156,11 @@ static int pairChunkEntries(long long entries) {
 }
 
 void PairScratch::release() {
-    if (base)
+    if (base && owned)
         cudaFree(base);
     base = nullptr;
     bytes = 0;
+    owned = false;
 }
 
 size_t PairScratch::bytesFor(const FrameJob *jobs, int n) {
@@ -1147,6 +1180,7 @@ bool PairScratch::reserve(size_t need) {
         return false;
     }
     bytes = need;
+    owned = true;
     // as for new workspaces (makeWorkspace)
     if (const char *e = std::getenv("LGCR_POISON_WORKSPACE"); e && e[0] == '1')
         cudaMemset(base, 0xFF, bytes);

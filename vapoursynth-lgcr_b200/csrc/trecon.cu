@@ -321,7 +321,7 @@ int lgcr_trecon_frame(lgcr_trecon *t, const lgcr_plane cur[3], const lgcr_plane 
         setError("TRecon: failed to upload geometry tables");
         return LGCR_E_NOMEM;
     }
-    Workspace *ws = F.acquire(true);
+    Workspace *ws = F.acquire(true, &task);
     if (!ws) {
         setError("TRecon: device workspace allocation failed");
         return LGCR_E_NOMEM;
