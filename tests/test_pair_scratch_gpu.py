@@ -106,3 +106,20 @@ def test_chunks_give_the_same_samples(kernel, fmt):
     for k, out in enumerate(mixed):
         for p in range(3):
             assert bool((alone[k % 3][p] == out[p]).all())
+
+
+@pytest.mark.parametrize("kernel", [dict(kernel="lanczos", taps=3, algo=2), dict(kernel="jinc", taps=3, algo=4)])
+def test_more_frames_than_one_prefix_table(kernel):
+    """A launch of more frames than a block's table of list lengths holds
+    (1024): the frames past it continue the entries of those before."""
+    w, h, n = 66, 34, 1030
+    rec = lgcr.Recon(lgcr.video_format(w, h, 10, 1, 1), **dict(kernel, sparse=0))
+    some = [device(S.make_frame(w, h, S.YUV420P10, seed=70 + k)) for k in range(3)]
+    alone, mixed = [outputs(rec, f) for f in some], [outputs(rec, some[0]) for _ in range(n)]
+    single = [run_batch([rec], [f], [o])[1][0] for f, o in zip(some, alone)][0]
+    _, launches = run_batch([rec] * n, [some[k % 3] for k in range(n)], mixed)
+    # the guided stage's one launch becomes two or three
+    assert launches == [single + (2 if kernel["kernel"] == "jinc" else 1)] * 2
+    for k, out in enumerate(mixed):
+        for p in range(3):
+            assert bool((alone[k % 3][p] == out[p]).all())

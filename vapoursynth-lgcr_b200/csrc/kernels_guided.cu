@@ -425,6 +425,7 @@ __device__ __forceinline__ void pairColumns(const FrameJob &J, uint32_t e, int &
 struct ExtremaWork {
     static __device__ __forceinline__ bool mine(const FrameJob &J) { return J.pairSup > 0 && J.radial; }
     static constexpr int kPer = 1;                       // threads per list entry
+    static constexpr bool kEndShared = true;             // the loop's end is read again (pairGrid)
     static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx, unsigned slot) {
         int ox, oy;
         bool on[2];
@@ -484,6 +485,7 @@ struct ExtremaWork {
 struct SetupWork {
     static __device__ __forceinline__ bool mine(const FrameJob &J) { return J.pairSup > 0; }
     static constexpr int kPer = 2;
+    static constexpr bool kEndShared = false;
     static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx, unsigned slot) {
         const uint32_t e = __ldg(J.actList + (idx >> 1));
         const int ox = (int)(e & 0xfffeu) + (int)(idx & 1u), oy = (int)(e >> 16);
@@ -601,6 +603,7 @@ struct PairWork {
         return J.pairSup > 0 && (J.radial != 0) == RADIAL;
     }
     static constexpr int kPer = 1;
+    static constexpr bool kEndShared = RADIAL;
     static __device__ __forceinline__ void run(const FrameJob &J, unsigned long long idx, unsigned slot) {
         int ox, oy;
         bool on[2];
@@ -782,10 +785,15 @@ __device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int 
     __shared__ unsigned long long pre[kPairMaxFrames + 1];
     __shared__ FrameJob sJob;
     __shared__ int sChunk;
+    __shared__ unsigned long long sEnd;
     const int tid = threadIdx.x;
-    unsigned long long before = 0;                       // threads of the frames before this part
+    if (tid == 0)
+        pre[0] = 0ull;
     for (int chunk = 0; chunk < njobs; chunk += kPairMaxFrames) {
         const int n = min(kPairMaxFrames, njobs - chunk);
+        __syncthreads();
+        if (tid == 0 && chunk > 0)
+            pre[0] = pre[kPairMaxFrames];                // after the frames before this part
         __syncthreads();
         for (int i = tid; i < n; i += kPairThreads) {
             const FrameJob &J = jobs[chunk + i];
@@ -795,20 +803,23 @@ __device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int 
         }
         __syncthreads();
         if (tid == 0) {
-            unsigned long long acc = before;
-            pre[0] = before;
+            unsigned long long acc = pre[0];
             for (int i = 1; i <= n; ++i)
                 pre[i] = acc += pre[i];
+            sEnd = min(acc, (first + (unsigned)sChunk) * Work::kPer);
         }
         __syncthreads();
-        const unsigned long long base = first * Work::kPer;
-        const unsigned long long begin = max(pre[0], base);
-        const unsigned long long total = before = pre[n];
-        const unsigned long long end = min(total, base + (unsigned long long)sChunk * Work::kPer);
         int staged = -1, f = 0;
-        for (unsigned long long lo = begin + (unsigned long long)blockIdx.x * kPairThreads; lo < end;
-             lo += (unsigned long long)gridDim.x * kPairThreads) {
-            const unsigned long long hi = min(lo + kPairThreads, end);
+        // jinc work has no register left for the end (held there, the extrema
+        // spill: 387 -> 406 us on one 4K frame); separable work does (reading
+        // it each time: one dense 1438x1079 4:2:2 frame 311 -> 319 us)
+        const unsigned long long held = sEnd;
+        const volatile unsigned long long &shared = sEnd;
+        auto end = [&] { return Work::kEndShared ? shared : held; };
+        for (unsigned long long lo = max(pre[0], first * Work::kPer) +
+                                     (unsigned long long)blockIdx.x * kPairThreads;
+             lo < end(); lo += (unsigned long long)gridDim.x * kPairThreads) {
+            const unsigned long long hi = min(lo + kPairThreads, end());
             while (pre[f + 1] <= lo)
                 ++f;
             for (int g = f; g < n && pre[g] < hi; ++g) {
@@ -823,7 +834,7 @@ __device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int 
                 }
                 const unsigned long long w = lo + tid;
                 if (w >= pre[g] && w < pre[g + 1] && w < hi)
-                    Work::run(sJob, w - pre[g], (unsigned)(w - base));
+                    Work::run(sJob, w - pre[g], (unsigned)(w - first * Work::kPer));
             }
         }
     }
