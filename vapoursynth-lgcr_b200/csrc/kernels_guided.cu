@@ -34,9 +34,8 @@
 // SM measured within 5 % of each other for k_guided_pair, 6 blocks 7 % better
 // than 4 for k_guided_pair_r; one merged kernel was slower than the pixel form
 // on separable frames. shapeJobs has the sizes from which this form is taken.
-// The assembler fuses a packed product and the packed sum that follows into
-// one fma, whatever -fmad says; the expressions here are written as the fmas
-// that the one-pixel kernel's packed loop becomes, so both give the same bits.
+// Both forms write the fused products of the packed tap arithmetic out as
+// fma2, the same ones, so both give the same bits.
 #include "guided.cuh"
 
 namespace lgcr_b200 {

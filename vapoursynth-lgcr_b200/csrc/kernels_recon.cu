@@ -782,8 +782,9 @@ k_plain_all(LGCR_STAGE_ARGS) {
 // Separable base weights, all taps in range, support SUP (even; fully
 // unrolled). The per-column products dx*nx and (-dx)*ny stay in registers;
 // columns are processed in pairs with tapCore's arithmetic on packed pairs
-// (range checks of the reciprocals hoisted by the caller), and each active
-// tap is accumulated in FP64 in tap order.
+// (range checks of the reciprocals hoisted by the caller; products and sums
+// fused as in the column pairs' taps, kernels_guided.cu), and each active tap
+// is accumulated in FP64 in tap order.
 // lc0/uv0 point at the window's tap (0, 0); rows are `stride` samples apart.
 // SH: the window was staged in shared memory by the warp (plain loads);
 // otherwise it is read from the planes in global memory.
@@ -823,7 +824,7 @@ __device__ __forceinline__ void tapsSeparable(const TapCtx &c, int tx0, int ty0,
     }
     const f32x2 one = pk2(1.0f, 1.0f);
     const f32x2 L0 = pk2(c.L0, c.L0), invS = pk2(c.invSigma2, c.invSigma2);
-    const f32x2 fade = pk2(c.guideFade, c.guideFade), resc = pk2(c.rescue, c.rescue);
+    const f32x2 nfade = pk2(-c.guideFade, -c.guideFade), resc = pk2(c.rescue, c.rescue);
     const f32x2 g2 = pk2(c.invG2, c.invG2), g2p = pk2(c.invG2Par, c.invG2Par);
 #pragma unroll
     for (int j = 0; j < SUP; ++j) {
@@ -843,19 +844,19 @@ __device__ __forceinline__ void tapsSeparable(const TapCtx &c, int tx0, int ty0,
             const double2 p1 = SH ? uvrow[i + 1] : __ldg(uvrow + i + 1);
             const float l0 = SH ? lrow[i] : ldf(lrow + i), l1 = SH ? lrow[i + 1] : ldf(lrow + i + 1);
             const f32x2 dL = sub2(pk2(l0, l1), L0);
-            const f32x2 simRaw = rcp2(add2(one, mul2(mul2(dL, dL), invS)), one);
-            const f32x2 sim = sub2(one, mul2(fade, sub2(one, simRaw)));
+            const f32x2 simRaw = rcp2(fma2(mul2(dL, dL), invS, one), one);
+            const f32x2 sim = fma2(nfade, sub2(one, simRaw), one);
             const f32x2 dp = add2(dxnx[q], dyny);
             const f32x2 dt = add2(dxny[q], dynx);
-            const f32x2 bump = rcp2(add2(add2(one, mul2(mul2(dp, dp), g2)), mul2(mul2(dt, dt), g2p)), one);
-            f32x2 base;
+            const f32x2 bump = rcp2(fma2(mul2(dt, dt), g2p, fma2(mul2(dp, dp), g2, one)), one);
+            f32x2 base;                                  // with the rescue term
             if (RADIAL) {
                 const float2 r2 = __ldg(radRow + q);
-                base = pk2(r2.x, r2.y);
+                base = fma2(resc, bump, pk2(r2.x, r2.y));
             } else {
-                base = mul2(wxv[q], wyy);
+                base = fma2(wxv[q], wyy, mul2(resc, bump));
             }
-            const f32x2 w = mul2(sim, add2(base, mul2(resc, bump)));
+            const f32x2 w = mul2(sim, base);
             float w0, w1;
             up2(w, w0, w1);
             if ((mx >> i) & 1u)

@@ -7,9 +7,10 @@
 // batched form); a block finds its frame by binary search over the prefix.
 //
 // Arithmetic in these kernels follows the reference's scalar build operation
-// by operation (the library is compiled with -fmad=false, so no product is
-// fused into an add unless written as an fma whose result is provably the
-// same). The device helpers restate:
+// by operation: the library is compiled with -fmad=false, so no scalar product
+// is fused into an add unless written as an fma whose result is provably the
+// same. Packed products are the exception (see f32x2 below). The device
+// helpers restate:
 //   bilinear / bilinearFast          src/lgcr.h:467-508
 //   principalTensorDirection         src/lgcr.h:516-538
 //   lutLookup                        src/lgcr.h:636-641
@@ -281,8 +282,12 @@ __device__ __forceinline__ float rcpAtLeastOne(float x) {
     return rcpOutOfRange(x);
 }
 
-// Two lanes of FP32 arithmetic per instruction: the packed f32x2 add, sub,
-// mul and fma of sm_100 round each lane exactly like the scalar instruction.
+// Two lanes of FP32 arithmetic per instruction: each packed f32x2 add, sub,
+// mul and fma of sm_100 rounds its lanes like the scalar instruction. The
+// assembler may make one fma of a packed product and the packed sum that takes
+// it, whatever -fmad says: one rounding instead of two. Where two kernels
+// evaluate the same expression (the guided taps) it is written as fma2, so
+// that the result does not depend on what the assembler makes of each.
 typedef unsigned long long f32x2;
 
 __device__ __forceinline__ f32x2 pk2(float a, float b) {
