@@ -198,6 +198,13 @@ int lgcr_debug_axis(const lgcr_recon *filter, int axis, double shift, int *start
  * reference (its divides are plain C++). */
 int lgcr_selftest_reciprocal(uint64_t *mismatches);
 
+/* Self-check of the quotients that are formed from a reciprocal, on the
+ * current device, bit for bit against the division: mismatches[0] the FP64
+ * quotients of a common denominator (2^30 seeded pairs), mismatches[1]
+ * Downsample's range weight of integer samples (every float of its range).
+ * 0 and 0 expected. No counterpart in the reference. */
+int lgcr_selftest_quotients(uint64_t mismatches[2]);
+
 /* ---------------------------------------------------------------------
  * Sharpen: the reference's second filter, a 5x5 gated bilateral unsharp
  * mask (luma self-guided; subsampled chroma guided by the sharpened luma's

@@ -189,15 +189,11 @@ k_yc_tiled(LGCR_STAGE_ARGS) {
     }
 }
 
-// Quotients n / d of one denominator, from its correctly rounded reciprocal r:
-// n * r corrected by its exact remainder is the IEEE quotient (Markstein, IBM
-// J. Res. Dev. 34(1), 1990), or NaN where n or n * r is not finite, and that
-// takes the division itself (out of line: its code and registers stay out of
-// the caller).
+// n / d by quotientBy; what it leaves (NaN) takes the division itself (out of
+// line: its code and registers stay out of the caller).
 __device__ __noinline__ double quotientCold(double n, double d) { return n / d; }
-__device__ __forceinline__ double quotientBy(double n, double d, double r) {
-    const double q = n * r;
-    const double v = fma(fma(-d, q, n), r, q);
+__device__ __forceinline__ double quotientOrDivide(double n, double d, double r) {
+    const double v = quotientBy(n, d, r);
     if (v == v)
         return v;
     return quotientCold(n, d);
@@ -264,7 +260,7 @@ __device__ __forceinline__ void affineSample(const FrameJob &J, int x, int y, bo
     const double eps = J.lgfEps;
     const double epsSig = J.epsSig;
     const double inv = 1.0 / n;
-    auto mean = [&](double sum) { return sparseRoi ? sum * inv : quotientBy(sum, (double)n, inv); };
+    auto mean = [&](double sum) { return sparseRoi ? sum * inv : quotientOrDivide(sum, (double)n, inv); };
     const double meanU = mean(s[0]), meanV = mean(s[2]);
     const double varU = smax(0.0, mean(s[1]) - meanU * meanU);
     const double varV = smax(0.0, mean(s[3]) - meanV * meanV);

@@ -38,7 +38,6 @@ __constant__ DsDirection kDsDirections[8] = {
 };
 
 constexpr float kDsActivation = 1.0e-4f;     // guidedActivationThreshold
-constexpr float kDsRangeScale2 = 2.25e-4f;   // accumulateGuided rangeScale2
 
 // one output block: 32 x 8 chroma samples; its source tile covers every
 // sample classify and accumulateGuided read (x in [2x - 4, 2x + 4], y in
@@ -190,16 +189,11 @@ __device__ DsStats dsClassify(const DsTile &T, float centerX, float centerY, int
     return st;
 }
 
-// kDsRangeScale2 / d for kDsRangeScale2 <= d: a refined reciprocal and
-// Markstein's remainder step (IBM J. Res. Dev. 34(1), 1990), the IEEE
-// quotient for finite d; float formats, whose d may overflow, divide.
+// Range weight; d is below 8 for integer samples, float samples may reach
+// infinity and divide.
 template <int KIND>
 __device__ __forceinline__ float dsRange(float d) {
-    if (KIND == kF32)
-        return kDsRangeScale2 / d;
-    const float r = rcpInRange(d);
-    const float q = kDsRangeScale2 * r;
-    return __fmaf_rn(__fmaf_rn(-q, d, kDsRangeScale2), r, q);
+    return KIND == kF32 ? kDownRangeScale2 / d : downRangeWeight(d);
 }
 
 // accumulateGuided (downsample.cpp:404-451): range- and spatially-weighted
@@ -233,7 +227,7 @@ __device__ __forceinline__ void dsAccumulate(const DownsampleJob &J, const DsTil
         for (int i = 0; i < J.winW; ++i, w += kDsSlots) {
             const int o = row + i;
             const float delta = T.y[o] - centerLuma;
-            const float rangeWeight = dsRange<KIND>(kDsRangeScale2 + delta * delta);
+            const float rangeWeight = dsRange<KIND>(kDownRangeScale2 + delta * delta);
             const float su = T.u[o], sv = T.v[o];
             const bool in = SMALL == 0 ||
                 (rowIn && fabsf((float)(J.winX0 + i) - (0.5f + J.shiftX)) <= 3.0f);

@@ -93,24 +93,6 @@ __device__ __noinline__ float probeClamped(const float *p, int w, int h, float x
     return bilinearAt(p, w, h, x, y);
 }
 
-// Quotients n0/d and n1/d for 1e-6 < d: one reciprocal refined to double
-// precision, then Markstein's remainder step per quotient (IBM J. Res. Dev.
-// 34(1), 1990).
-__device__ __forceinline__ void divide2(double n0, double n1, double d, double &q0, double &q1) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    double e = fma(-d, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-d, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-d, r, 1.0);
-    r = fma(r, e, r);
-    q0 = n0 * r;
-    q1 = n1 * r;
-    q0 = fma(fma(-q0, d, n0), r, q0);
-    q1 = fma(fma(-q1, d, n1), r, q1);
-}
-
 // Context of one listed pixel (k_guide_setup to k_guided_pair): two float4 at
 // 2 * (entry's place in the chunk) + column.
 //   a = (L0, nx, ny, 1/sigma^2), the last negative when a similarity
@@ -727,7 +709,9 @@ struct PairWork {
             double valueU, valueV;
             if (good[q]) {
                 if (J.inKind != kF32) {
-                    divide2(sums[q].u, sums[q].v, sums[q].wsum, valueU, valueV);
+                    const double r = __drcp_rn(sums[q].wsum);
+                    valueU = quotientBy(sums[q].u, sums[q].wsum, r);
+                    valueV = quotientBy(sums[q].v, sums[q].wsum, r);
                 } else {                                 // float samples may be infinite
                     valueU = sums[q].u / sums[q].wsum;
                     valueV = sums[q].v / sums[q].wsum;

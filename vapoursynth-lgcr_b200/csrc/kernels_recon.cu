@@ -218,21 +218,18 @@ struct PlainRows {
 };
 
 // The pixel's value from its vertical sums: normalised, or bilinear where the
-// weights cancel, then held to the hull. One correctly rounded reciprocal
-// serves U and V: n * r corrected by its exact remainder is the IEEE quotient
-// (Markstein, IBM J. Res. Dev. 34(1), 1990), or NaN where n or n * r is not
-// finite, and those take the division (ws, a product of two floats above 1e-6,
-// has a normal reciprocal). The hull bounds are floats and rounding is
-// monotone, so the clamp runs on the rounded value.
+// weights cancel, then held to the hull. One reciprocal serves U and V
+// (quotientBy; ws, a product of two floats above 1e-6, has a normal one), and
+// what it leaves takes the division. The hull bounds are floats and rounding
+// is monotone, so the clamp runs on the rounded value.
 __device__ __forceinline__ float2 plainValue(const FrameJob &J, double vU, double vV, float mnU, float mxU,
                                              float mnV, float mxV, double ws, double wa, float posX,
                                              float posY) {
     float u, v;
     if (ws > 1e-6 && ws >= 0.05 * wa) {
         const double r = __drcp_rn(ws);
-        const double qU = vU * r, qV = vV * r;
-        u = (float)fma(fma(-ws, qU, vU), r, qU);
-        v = (float)fma(fma(-ws, qV, vV), r, qV);
+        u = (float)quotientBy(vU, ws, r);
+        v = (float)quotientBy(vV, ws, r);
         if (u != u || v != v) {
             u = (float)(vU / ws);
             v = (float)(vV / ws);

@@ -267,8 +267,8 @@ constexpr float kRcpFastLimit = 18446744073709551616.0f;   // 2^64
 // of line so the unrolled tap loops that call rcpAtLeastOne stay compact.
 static __device__ __noinline__ float rcpOutOfRange(float x) { return 1.0f / x; }
 
-// The refinement alone, for callers that have shown x < 2^64 (or NaN, which
-// it returns as the division would).
+// The refinement alone, for callers that have shown 1 <= x < 2^64 (or NaN,
+// which it returns as the division would).
 __device__ __forceinline__ float rcpInRange(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -280,6 +280,25 @@ __device__ __forceinline__ float rcpAtLeastOne(float x) {
     if (x < kRcpFastLimit)
         return rcpInRange(x);
     return rcpOutOfRange(x);
+}
+
+// n / d from r = __drcp_rn(d), for several quotients of one denominator: the
+// product n * r corrected by its exact remainder (Markstein, IBM J. Res. Dev.
+// 34(1), 1990), or NaN where n or n * r is not finite. lgcr_selftest_quotients
+// finds no difference from the division over the range in use.
+__device__ __forceinline__ double quotientBy(double n, double d, double r) {
+    const double q = n * r;
+    return fma(fma(-d, q, n), r, q);
+}
+
+// kDownRangeScale2 / d for kDownRangeScale2 <= d < 8 (Downsample's range weight
+// of integer samples): the same correction of a refined reciprocal, compared
+// with the division for every such float by lgcr_selftest_quotients.
+constexpr float kDownRangeScale2 = 2.25e-4f;  // accumulateGuided rangeScale2, src/downsample.cpp
+__device__ __forceinline__ float downRangeWeight(float d) {
+    const float r = rcpInRange(d);
+    const float q = kDownRangeScale2 * r;
+    return __fmaf_rn(__fmaf_rn(-q, d, kDownRangeScale2), r, q);
 }
 
 // Two lanes of FP32 arithmetic per instruction: each packed f32x2 add, sub,
