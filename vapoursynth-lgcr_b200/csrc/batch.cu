@@ -55,6 +55,7 @@ struct lgcr_batch {
     PairScratch pairs;
     int pairsSlot = -1;
     int lastLaunches = 0;
+    bool lastPixelForm = false;         // a listed frame of the last run took the pixel form
     // profiling
     bool profiling = false;
     std::vector<StageEvent> events;
@@ -408,6 +409,9 @@ int lgcr_batch_run(lgcr_batch *b, const lgcr_batch_item *items, int count, void 
         }
     }
     b->lastLaunches = launches;
+    b->lastPixelForm = false;
+    for (const FrameJob &J : jobs)
+        b->lastPixelForm = b->lastPixelForm || (J.listed && J.pairSup == 0);
     cudaEventRecord(sl.done, s);
     sl.pending = true;
     b->next = (b->next + 1) % kDescriptorSlots;
@@ -504,7 +508,7 @@ extern "C" int lgcr_autotune(const lgcr_batch_item *items, int count, void *stre
             text += line + buf;
         }
     }
-    // register budget of the persistent guided stage
+    // register budget of the persistent guided stage's pixel form
     if (status == LGCR_OK) {
         int guidedStage = -1;
         for (int s = 0; s < stageCount(); ++s)
@@ -523,6 +527,10 @@ extern "C" int lgcr_autotune(const lgcr_batch_item *items, int count, void *stre
             lgcr_batch_stage_times(b, ms.data(), nullptr, 1);
             if (ms[guidedStage] <= 0.0)
                 break;
+            if (!b->lastPixelForm) {           // the variants are the pixel form's
+                text += line + " column pairs\n";
+                break;
+            }
             char buf[64];
             std::snprintf(buf, sizeof(buf), " %s=%.3fms", names[v], ms[guidedStage] / 2);
             line += buf;
@@ -545,7 +553,8 @@ extern "C" int lgcr_autotune(const lgcr_batch_item *items, int count, void *stre
 // settings, so other batches and per-frame calls keep running unchanged:
 //  * the block shape of every tunable per-pixel stage the items use
 //    (stage-event time of that stage);
-//  * the persistent guided kernel's variant (its stage-event time);
+//  * the persistent guided kernel's variant (its stage-event time), where a
+//    frame of the layout takes the pixel form, whose variants they are;
 //  * the frame grouping of the stage sequence (whole-run time, events around
 //    three runs): upscaling frames alone, one group, or one frame per group.
 // Later runs of this batch plan with the chosen settings and re-capture their
@@ -618,6 +627,10 @@ extern "C" int lgcr_batch_autotune(lgcr_batch *b, const lgcr_batch_item *items, 
             stageRun();
             if (status != LGCR_OK || ms[guidedStage] <= 0.0)
                 break;
+            if (!b->lastPixelForm) {            // the variants are the pixel form's
+                text += line + " column pairs\n";
+                break;
+            }
             char buf[64];
             std::snprintf(buf, sizeof(buf), " %s=%.3fms", variantNames[v], ms[guidedStage]);
             line += buf;
