@@ -123,3 +123,35 @@ def test_more_frames_than_one_prefix_table(kernel):
     for k, out in enumerate(mixed):
         for p in range(3):
             assert bool((alone[k % 3][p] == out[p]).all())
+
+
+def test_a_growing_batch():
+    """One batch object meeting larger and larger launches: its scratch grows
+    in powers of two, and the samples stay those of a launch alone."""
+    lib = lgcr.library()
+    rec = lgcr.Recon(lgcr.video_format(640, 360, 10, 1, 1), kernel="lanczos", taps=3, algo=2)
+    frame = device(S.make_frame(640, 360, S.YUV420P10, seed=12))
+    outs = [outputs(rec, frame) for _ in range(24)]
+    alone = rec.frame(frame, -1, out=outputs(rec, frame))
+    items = (lgcr.BatchItem * len(outs))()
+    for i, out in enumerate(outs):
+        items[i].filter = rec.handle
+        items[i].inp = lgcr.planes_desc(frame)
+        items[i].out = lgcr.planes_desc(out)
+        items[i].chroma_location = -1
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    handle = ctypes.c_void_p()
+    assert lib.lgcr_batch_create(ctypes.byref(handle)) == 0
+    for n in range(1, len(outs) + 1):           # 0.2 to 5.5 million pixels: pairs from 7 frames on
+        for out in outs[:n]:
+            for p in out:
+                p.zero_()
+        stream.wait_stream(torch.cuda.current_stream())
+        assert lib.lgcr_batch_run(handle, items, n, ctypes.c_void_p(stream.cuda_stream), n % 2) == 0, \
+            lib.lgcr_last_error().decode()
+        stream.synchronize()
+        for out in outs[:n]:
+            for p in range(3):
+                assert bool((out[p] == alone[p]).all()), (n, p)
+    lib.lgcr_batch_destroy(handle)

@@ -112,7 +112,8 @@ struct PairScratch {
     ~PairScratch() { release(); }
     // What the launch of these shaped jobs takes (0: no frame takes pairs).
     static size_t bytesFor(const FrameJob *jobs, int n);
-    // Grows to `need` bytes. Work that uses the scratch must have ended.
+    // Grows to `need` bytes or more (less than 1 GiB). Work that uses the
+    // scratch must have ended.
     bool reserve(size_t need);
     // Gives the jobs of one launch the scratch; where it could not be had they
     // take the pixel form, which needs none.

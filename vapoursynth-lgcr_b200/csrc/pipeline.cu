@@ -1173,13 +1173,20 @@ size_t PairScratch::bytesFor(const FrameJob *jobs, int n) {
 bool PairScratch::reserve(size_t need) {
     if (need <= bytes)
         return true;
+    // a scratch that grows again does so in powers of two, since each growth
+    // synchronizes the device (a serving lane meets larger and larger mixes)
+    size_t size = need;
+    if (bytes > 0)
+        for (size = 1 << 20; size < need; size *= 2) {}
     release();
-    if (cudaMalloc(&base, need) != cudaSuccess) {
+    if (cudaMalloc(&base, size) != cudaSuccess) {
         cudaGetLastError();                            // not this call's error: it has another way
         base = nullptr;
-        return false;
+        if (size == need)
+            return false;
+        return reserve(need);
     }
-    bytes = need;
+    bytes = size;
     owned = true;
     // as for new workspaces (makeWorkspace)
     if (const char *e = std::getenv("LGCR_POISON_WORKSPACE"); e && e[0] == '1')
