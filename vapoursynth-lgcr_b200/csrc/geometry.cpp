@@ -7,7 +7,6 @@
 #include <cmath>
 #include <cstring>
 #include <string>
-#include <string>
 #include <unordered_map>
 
 namespace lgcr_b200 {

@@ -181,7 +181,7 @@ __device__ __forceinline__ void pairTaps(const FrameJob &J, const Pair &c, int o
                     const float2 r = __ldg(rad + j * UC + i);
                     base = pk2(__fmaf_rn(-c.rescue[0], nb, r.x), r.y);
                 } else {
-                        base = pk2(__fmaf_rn(t.x, wy, -c.rescue[0] * nb), t.y * wy);
+                    base = pk2(__fmaf_rn(t.x, wy, -c.rescue[0] * nb), t.y * wy);
                 }
             }
             float w0, w1;
@@ -377,11 +377,6 @@ __device__ __noinline__ void selectPixel(const FrameJob &J, int ox, int oy, cons
 struct PairTables {
     int ox;
     bool two;
-    __device__ __forceinline__ int2 i2(const int *t) const {
-        int2 v = __ldg(reinterpret_cast<const int2 *>(t + ox));
-        if (!two) v.y = v.x;
-        return v;
-    }
     __device__ __forceinline__ float2 f2(const float *t) const {
         float2 v = __ldg(reinterpret_cast<const float2 *>(t + ox));
         if (!two) v.y = v.x;
