@@ -29,8 +29,8 @@
 //    the kernel's own negative weight, and a pair that the bound does not
 //    clear is evaluated again with the sum.
 // Measured: 1080p lanczos4 4:2:0 (55 % listed) 202 us for the one-pixel kernel,
-// 53 + 129 here; 1080p -> 4K jinc selector, 16-bit, 1800 us before, 387
-// (extrema) + 312 (setup) + 764 (pairs). Register budgets of 4 to 8 blocks per
+// 53 + 129 here; 1080p -> 4K jinc selector, 16-bit, 1800 us before, 392
+// (extrema) + 312 (setup) + 766 (pairs). Register budgets of 4 to 8 blocks per
 // SM measured within 5 % of each other for k_guided_pair, 6 blocks 7 % better
 // than 4 for k_guided_pair_r; one merged kernel was slower than the pixel form
 // on separable frames. shapeJobs has the sizes from which this form is taken.
@@ -789,8 +789,8 @@ __device__ __forceinline__ void pairGrid(const FrameJob *__restrict__ jobs, int 
         __syncthreads();
         int staged = -1, f = 0;
         // jinc work has no register left for the end (held there, the extrema
-        // spill: 387 -> 406 us on one 4K frame); separable work does (reading
-        // it each time: one dense 1438x1079 4:2:2 frame 311 -> 319 us)
+        // spill: 406 us on one 4K frame, 392 read from shared memory); separable
+        // work does (one dense 1438x1079 4:2:2 frame 311 us, 319 with the read)
         const unsigned long long held = sEnd;
         const volatile unsigned long long &shared = sEnd;
         auto end = [&] { return Work::kEndShared ? shared : held; };
